@@ -433,18 +433,16 @@ __global__ void __launch_bounds__(32 * SEG) k_sweep_batch_part(NDBatch B, long s
         };
         // downward
         int p = s0 + 1;
-        double inv = rcp_full(brow(p));
         double a = arow(p);
-        double alp = a * inv, gap = crow(p) * inv, dep = tile[p * tp + t] * inv;
+        double alp, gap, dep;
+        pivot3(brow(p), a, crow(p), tile[p * tp + t], alp, gap, dep);
         al[p * nt + t] = alp;
         ga[p * nt + t] = gap;
         tile[p * tp + t] = dep;
         for (p = s0 + 2; p < s0 + m; p++) {
             a = arow(p);
-            inv = rcp_full(fma(-a, gap, brow(p)));
-            alp = -a * alp * inv;
-            gap = crow(p) * inv;
-            dep = fma(-a, dep, tile[p * tp + t]) * inv;
+            pivot3(fma(-a, gap, brow(p)), -a * alp, crow(p), fma(-a, dep, tile[p * tp + t]), alp,
+                   gap, dep);
             al[p * nt + t] = alp;
             ga[p * nt + t] = gap;
             tile[p * tp + t] = dep;
@@ -467,10 +465,12 @@ __global__ void __launch_bounds__(32 * SEG) k_sweep_batch_part(NDBatch B, long s
         }
         // row 0 with x_1 substituted, solved for x_0
         const double c0 = crow(s0);
-        const double iB = rcp_full(fma(-c0, alu, brow(s0)));
-        r8[0] = arow(s0) * iB;
-        r8[1 * nt] = (-c0 * gau) * iB;
-        r8[2 * nt] = fma(-c0, deu, tile[s0 * tp + t]) * iB;
+        double xa, xc, xd;
+        pivot3(fma(-c0, alu, brow(s0)), arow(s0), -c0 * gau, fma(-c0, deu, tile[s0 * tp + t]), xa,
+               xc, xd);
+        r8[0] = xa;
+        r8[1 * nt] = xc;
+        r8[2 * nt] = xd;
     }
     __syncthreads();
     if (t < n) {
@@ -499,9 +499,7 @@ __global__ void __launch_bounds__(32 * SEG) k_sweep_batch_part(NDBatch B, long s
             const double *rr = red + (size_t)k * PART_SLOTS * nt + t;
             const double ra = rr[3 * nt], rb = rr[4 * nt], rc = rr[5 * nt], rd = rr[6 * nt];
             const double bet = (k == 0) ? rb : fma(-ra, g, rb);
-            const double iv = rcp_full(bet);
-            u = ((k == 0) ? rd : fma(-ra, u, rd)) * iv;
-            g = rc * iv;
+            pivot(bet, (k == 0) ? rd : fma(-ra, u, rd), rc, u, g);
             gm[k] = g;
             z[k] = u;
         }

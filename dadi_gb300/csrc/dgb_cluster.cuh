@@ -67,17 +67,15 @@ __device__ __forceinline__ void c2_sweep_x(cooperative_groups::cluster_group &cl
         };
         int p = 1;
         double aa = arow(R0 + p);
-        double inv = rcp_full(brow(R0 + p));
-        double alp = aa * inv, gap = crow(R0 + p) * inv, dep = blk[p * pitch + j] * inv;
+        double alp, gap, dep;
+        pivot3(brow(R0 + p), aa, crow(R0 + p), blk[p * pitch + j], alp, gap, dep);
         al[p * L + j] = alp;
         ga[p * L + j] = gap;
         blk[p * pitch + j] = dep;
         for (p = 2; p < m; p++) {
             aa = arow(R0 + p);
-            inv = rcp_full(fma(-aa, gap, brow(R0 + p)));
-            alp = -aa * alp * inv;
-            gap = crow(R0 + p) * inv;
-            dep = fma(-aa, dep, blk[p * pitch + j]) * inv;
+            pivot3(fma(-aa, gap, brow(R0 + p)), -aa * alp, crow(R0 + p),
+                   fma(-aa, dep, blk[p * pitch + j]), alp, gap, dep);
             al[p * L + j] = alp;
             ga[p * L + j] = gap;
             blk[p * pitch + j] = dep;
@@ -97,10 +95,11 @@ __device__ __forceinline__ void c2_sweep_x(cooperative_groups::cluster_group &cl
             ga[p * L + j] = gau;
         }
         const double c0 = crow(R0);
-        const double iB = rcp_full(fma(-c0, alu, brow(R0)));
-        xr[0 * L + j] = arow(R0) * iB;
-        xr[1 * L + j] = (-c0 * gau) * iB;
-        xr[2 * L + j] = fma(-c0, deu, blk[j]) * iB;
+        double xa, xc, xd;
+        pivot3(fma(-c0, alu, brow(R0)), arow(R0), -c0 * gau, fma(-c0, deu, blk[j]), xa, xc, xd);
+        xr[0 * L + j] = xa;
+        xr[1 * L + j] = xc;
+        xr[2 * L + j] = xd;
     }
     cluster.sync();
     if (j < L && j % S == rank) {
@@ -123,9 +122,7 @@ __device__ __forceinline__ void c2_sweep_x(cooperative_groups::cluster_group &cl
             const double rc = -gaq * Cn;
             const double rd = fma(-gaq, Dn, fma(-alq, Dp, deq));
             const double bet = (q == 0) ? rb : fma(-ra, gq, rb);
-            const double iv = rcp_full(bet);
-            u = ((q == 0) ? rd : fma(-ra, u, rd)) * iv;
-            gq = rc * iv;
+            pivot(bet, (q == 0) ? rd : fma(-ra, u, rd), rc, u, gq);
             gm[q] = gq;
             z[q] = u;
         }
@@ -179,17 +176,15 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
         };
         int c = s0 + 1;
         double aa = arow(c);
-        double inv = rcp_full(brow(c));
-        double alp = aa * inv, gap = crow(c) * inv, dep = ph[c] * inv;
+        double alp, gap, dep;
+        pivot3(brow(c), aa, crow(c), ph[c], alp, gap, dep);
         al[c * C2_ROWS + p] = alp;
         ga[c * C2_ROWS + p] = gap;
         ph[c] = dep;
         for (c = s0 + 2; c < s0 + ml; c++) {
             aa = arow(c);
-            inv = rcp_full(fma(-aa, gap, brow(c)));
-            alp = -aa * alp * inv;
-            gap = crow(c) * inv;
-            dep = fma(-aa, dep, ph[c]) * inv;
+            pivot3(fma(-aa, gap, brow(c)), -aa * alp, crow(c), fma(-aa, dep, ph[c]), alp, gap,
+                   dep);
             al[c * C2_ROWS + p] = alp;
             ga[c * C2_ROWS + p] = gap;
             ph[c] = dep;
@@ -209,10 +204,11 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
             ga[c * C2_ROWS + p] = gau;
         }
         const double c0 = crow(s0);
-        const double iB = rcp_full(fma(-c0, alu, brow(s0)));
-        r8[0] = arow(s0) * iB;
-        r8[1 * C2_ROWS] = (-c0 * gau) * iB;
-        r8[2 * C2_ROWS] = fma(-c0, deu, ph[s0]) * iB;
+        double xa, xc, xd;
+        pivot3(fma(-c0, alu, brow(s0)), arow(s0), -c0 * gau, fma(-c0, deu, ph[s0]), xa, xc, xd);
+        r8[0] = xa;
+        r8[1 * C2_ROWS] = xc;
+        r8[2 * C2_ROWS] = xd;
     }
     __syncthreads();
     if (live) {
@@ -240,9 +236,7 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
             const double ra = rr[3 * C2_ROWS], rb = rr[4 * C2_ROWS];
             const double rc = rr[5 * C2_ROWS], rd = rr[6 * C2_ROWS];
             const double bet = (k == 0) ? rb : fma(-ra, gq, rb);
-            const double iv = rcp_full(bet);
-            u = ((k == 0) ? rd : fma(-ra, u, rd)) * iv;
-            gq = rc * iv;
+            pivot(bet, (k == 0) ? rd : fma(-ra, u, rd), rc, u, gq);
             gm[k] = gq;
             z[k] = u;
         }

@@ -17,6 +17,8 @@
 //  * 1/bet uses the hardware reciprocal seed (rcp.approx.ftz.f64) refined by
 //    one third-order Newton-Raphson step r(1 + e + e^2), e = 1 - x r, which
 //    is accurate to about one ulp; quotients become products.
+//  * The reciprocal and the products with it are formed on the integer pipes
+//    (pivot, below), which leaves 5 of the 10 on the FP64 pipe.
 // These reassociations move results by a few ulps per step relative to the
 // reference C, far inside the 1e-9 relative bar on extrapolated spectra.
 //
@@ -51,12 +53,154 @@ __device__ __forceinline__ double rcp_seed(double x)
     return r;
 }
 
-// Reciprocal to ~1 ulp: seed refined by one cubic Newton-Raphson step.
-__device__ __forceinline__ double rcp_full(double x)
+// Reciprocal to ~1 ulp: seed refined by one cubic Newton-Raphson step.  Not
+// inlined: it is the rare other side of rcp_full and pivot below, and a
+// predicated-off FP64 instruction takes the pipe like one that runs.
+static __device__ __noinline__ double rcp_newton(double x)
 {
     double r = rcp_seed(x);
     double e = fma(-x, r, 1.0);
     return fma(r, fma(e, e, e), r);
+}
+
+// The same reciprocal, and products with it, on the integer pipes.
+//
+// The SM has one FP64 pipe: an FP64 instruction of a warp takes it 16 cycles
+// (64 issue slots of a sub-partition; DMUL and DADD 19), and one warp issues
+// at most one per 64 cycles.  A sweep is bound by its count of FP64
+// instructions, whatever their dependencies, while the integer pipes stand
+// idle.  So of the 10 FP64 instructions of a grid point the three of the
+// reciprocal and the products t * inv and c * inv are done with 32 x 32 -> 64
+// bit multiply-adds instead (about 110 instructions), which leaves 5.
+// Measured, Thomas lines of 48 points on one SM, cycles per point and warp of
+// lines: 171 -> 88 with 16 warps, 175 -> 110 with 7, 844 -> 634 for one warp
+// (its chain: 134 cycles for the reciprocal, 108 for a product).  1,000 IM
+// spectra at pts 80/90/100: 1.08 -> 0.73 s.  The
+// results are the same bits as those of rcp_newton and of IEEE multiplication:
+// every value is rounded from one that carries 32 or more further bits, and
+// where these cannot tell which way the rounding on doubles goes (one pivot
+// in 8,000), or a value leaves the range handled here, the doubles decide.
+//
+// rcp_mant: for x = m 2^E, X = m 2^52 (53 bits) and the seed r0 of 1/m as rho
+// = r0 2^21 (21 bits), -X rho mod 2^64 is the residual e = 1 - m r0 (|e| <
+// 2^-19) in units of 2^-73, exactly; then 1/m = r0 (1 + e + e^2) is built in
+// units of 2^-96 with an error below 2^-67, and rounded to 53 bits.
+struct Mant {
+    unsigned h, l; // 2^64 / m rounded to 53 bits: the top bit of h is set
+};
+
+__device__ __forceinline__ Mant rcp_mant(double x, bool &bad)
+{
+    const unsigned xh = (unsigned)__double2hiint(x), xl = (unsigned)__double2loint(x);
+    const unsigned hx = (xh & 0xfffffu) | 0x100000u;
+    const double seed = rcp_seed(__hiloint2double((int)(hx + 0x3fe00000u), (int)xl));
+    const unsigned rho = (unsigned)__double2hiint(seed) - 0x3fd00000u;
+    const unsigned nr = 0u - rho; // xl * nr counts xl 2^32 too much
+    const unsigned long long t = (unsigned long long)xl * nr;
+    const unsigned eh = (unsigned)(t >> 32) + hx * nr - xl;
+    const unsigned long long e = (unsigned long long)eh << 32 | (unsigned)t;
+    const int s = (int)__funnelshift_r((unsigned)t, eh, 23);
+    const unsigned long long f = (unsigned long long)(unsigned)__mulhi(s, s) * 32u + e;
+    const unsigned r4 = rho << 2;
+    const unsigned long long w = (unsigned long long)r4 * (unsigned)f;
+    const unsigned long long r =
+        (unsigned long long)((long long)(int)r4 * (int)(f >> 32)) +
+        ((unsigned long long)(rho << 11) << 32 | (unsigned)(w >> 32));
+    // the bits below the 53rd, against one half, within the error
+    const unsigned v = __funnelshift_l((unsigned)w, (unsigned)r, 21);
+    const unsigned long long y = r + 0x400u;
+    Mant o;
+    o.h = (unsigned)(y >> 32);
+    o.l = (unsigned)y & ~0x7ffu;
+    // (the top bit is clear for m = 1; exponents from -128 to 127)
+    bad = (v - 0x7ffc0000u < 0x80000u) | ((int)o.h >= 0) |
+          ((xh & 0x7fffffffu) - 0x37f00000u >= 0x10000000u);
+    return o;
+}
+
+// x * (1/b) for the mantissa y of 1/b, rounded as IEEE multiplication rounds;
+// exps = exponent field of 1/b less the bias and one.
+__device__ __forceinline__ double mul_mant(double x, const Mant &y, unsigned exps, bool &bad)
+{
+    const unsigned xh = (unsigned)__double2hiint(x), xl = (unsigned)__double2loint(x);
+    const unsigned mh = (xh & 0xfffffu) | 0x100000u;
+    const unsigned long long t1 = (unsigned long long)mh * y.l + __umulhi(xl, y.l);
+    const unsigned long long t2 = (unsigned long long)xl * y.h + (unsigned)t1;
+    const unsigned long long p = (unsigned long long)mh * y.h +
+                                 ((unsigned long long)(unsigned)(t1 >> 32) + (unsigned)(t2 >> 32));
+    const unsigned w1 = (unsigned)t2, w2 = (unsigned)p, w3 = (unsigned)(p >> 32);
+    const unsigned sh = (w3 >> 20) ^ 1u; // mantissa in [1, 2): one bit up
+    const unsigned m1 = w1 << sh;
+    const unsigned long long m = ((unsigned long long)__funnelshift_l(w2, w3, sh) << 32 |
+                                  __funnelshift_l(w1, w2, sh)) +
+                                 (m1 >> 31);
+    // (a tie, or a value whose product may leave the normal range)
+    bad = bad | (m1 == 0x80000000u) | ((xh & 0x7fffffffu) - 0x0c800000u >= 0x66000000u);
+    return __hiloint2double(
+        (int)((unsigned)(m >> 32) + (xh & 0xfff00000u) + exps + (w3 & 0x100000u)),
+        (int)(unsigned)m);
+}
+
+__device__ __forceinline__ unsigned rcp_exps(double x)
+{
+    return 0x3fd00000u - ((unsigned)__double2hiint(x) & 0xfff00000u);
+}
+
+__device__ __forceinline__ double rcp_full(double x)
+{
+    bool bad;
+    const Mant y = rcp_mant(x, bad);
+    double r = __hiloint2double((int)((y.h >> 11) + 0x3ff00000u + rcp_exps(x)),
+                                (int)__funnelshift_r(y.l, y.h, 11));
+    if (bad)
+        r = rcp_newton(x);
+    return r;
+}
+
+static __device__ __noinline__ double2 pivot_fp64(double bet, double t, double c)
+{
+    const double inv = rcp_newton(bet);
+    return make_double2(t * inv, c * inv);
+}
+
+// u = t * (1/bet) and g = c * (1/bet).
+__device__ __forceinline__ void pivot(double bet, double t, double c, double &u, double &g)
+{
+    bool bad;
+    const Mant y = rcp_mant(bet, bad);
+    const unsigned exps = rcp_exps(bet);
+    u = mul_mant(t, y, exps, bad);
+    g = mul_mant(c, y, exps, bad);
+    if (bad) {
+        const double2 ug = pivot_fp64(bet, t, c);
+        u = ug.x;
+        g = ug.y;
+    }
+}
+
+static __device__ __noinline__ double3 pivot3_fp64(double bet, double t, double c, double d)
+{
+    const double inv = rcp_newton(bet);
+    return make_double3(t * inv, c * inv, d * inv);
+}
+
+// u = t * (1/bet), g = c * (1/bet) and w = d * (1/bet): the rows of the
+// partitioned solves.
+__device__ __forceinline__ void pivot3(double bet, double t, double c, double d, double &u,
+                                       double &g, double &w)
+{
+    bool bad;
+    const Mant y = rcp_mant(bet, bad);
+    const unsigned exps = rcp_exps(bet);
+    u = mul_mant(t, y, exps, bad);
+    g = mul_mant(c, y, exps, bad);
+    w = mul_mant(d, y, exps, bad);
+    if (bad) {
+        const double3 r = pivot3_fp64(bet, t, c, d);
+        u = r.x;
+        g = r.y;
+        w = r.z;
+    }
 }
 
 // ------------------------------------------------------- parameter schedule
@@ -299,31 +443,26 @@ __device__ __forceinline__ void solve_line(TP *__restrict__ ph, int sp, TG *__re
                                            int gs, int L, double W, double bs, double be,
                                            const AxisVecs &v, const AxisScalars &s)
 {
-    double b = fma(W, s.B1s, v.B0[0]) + bs;
-    double inv = rcp_full(b);
-    double u = ph[0] * inv;
+    double u, g, none;
+    pivot(fma(W, s.B1s, v.B0[0]) + bs, ph[0], fma(W, v.C1[0], v.C0[0]), u, g);
     ph[0] = u;
-    double g = fma(W, v.C1[0], v.C0[0]) * inv;
     gm[gs] = g;
-    int i = 1;
-#pragma unroll 2
-    for (; i < L - 1; i++) {
-        double a = fma(W, v.A1[i], v.A0[i]);
-        double bet = fma(-a, g, v.B0[i]);
-        inv = rcp_full(bet);
-        u = fma(-a, u, ph[i * sp]) * inv;
+    // row i's coefficients and right-hand side are formed while row i - 1's
+    // pivot is still in the integer pipes
+    double a = fma(W, v.A1[1], v.A0[1]), c = fma(W, v.C1[1], v.C0[1]);
+    double b0 = v.B0[1], p = ph[sp];
+    for (int i = 1; i < L - 1; i++) {
+        const double bet = fma(-a, g, b0), t = fma(-a, u, p), ci = c;
+        a = fma(W, v.A1[i + 1], v.A0[i + 1]);
+        c = fma(W, v.C1[i + 1], v.C0[i + 1]);
+        b0 = v.B0[i + 1];
+        p = ph[(i + 1) * sp];
+        pivot(bet, t, ci, u, g);
         ph[i * sp] = u;
-        g = fma(W, v.C1[i], v.C0[i]) * inv;
         gm[(i + 1) * gs] = g;
     }
-    {
-        double a = fma(W, v.A1[i], v.A0[i]);
-        double bl = fma(W, s.B1e, v.B0[i]) + be;
-        double bet = fma(-a, g, bl);
-        inv = rcp_full(bet);
-        u = fma(-a, u, ph[i * sp]) * inv;
-        ph[i * sp] = u;
-    }
+    pivot(fma(-a, g, fma(W, s.B1e, b0) + be), fma(-a, u, p), 1.0, u, none);
+    ph[(L - 1) * sp] = u;
     back_substitute(ph, sp, gm, gs, L, u);
 }
 

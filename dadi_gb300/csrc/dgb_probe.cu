@@ -31,6 +31,21 @@ __global__ void k_rcp(const double *x, double *out, int n)
     if (i < n)
         out[i] = rcp_full(x[i]);
 }
+// u = t * (1/x), g = c * (1/x) by pivot and, after them, on doubles.
+__global__ void k_pivot(const double *xtc, double *out, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n)
+        return;
+    const double x = xtc[i], t = xtc[(size_t)n + i], c = xtc[2 * (size_t)n + i];
+    double u, g;
+    pivot(x, t, c, u, g);
+    const double2 d = pivot_fp64(x, t, c);
+    out[i] = u;
+    out[(size_t)n + i] = g;
+    out[2 * (size_t)n + i] = d.x;
+    out[3 * (size_t)n + i] = d.y;
+}
 } // namespace dgb
 
 extern "C" int dgb_probe_fp64_fma(double *out, int blocks, int threads, int iters,
@@ -53,6 +68,16 @@ extern "C" int dgb_probe_rcp(const double *x, double *out, int n, void *stream)
     return cudaGetLastError() == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
 }
 
+extern "C" int dgb_probe_pivot(const double *xtc, double *out, int n, void *stream)
+{
+    if (!xtc || !out || n < 0)
+        return DGB_ERR_ARG;
+    if (n == 0)
+        return DGB_OK;
+    dgb::k_pivot<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(xtc, out, n);
+    return cudaGetLastError() == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
+}
+
 namespace dgb {
-int preload_probe() { return preload(k_fp64_fma) + preload(k_rcp); }
+int preload_probe() { return preload(k_fp64_fma) + preload(k_rcp) + preload(k_pivot); }
 } // namespace dgb

@@ -185,17 +185,14 @@ __global__ void k_precalc_nd(NDArgs A)
         double *gm = gam + t;
         const double *a = A.ca + base, *b = A.cb + base, *c = A.cc + base;
         const long S = A.S;
-        double bet = b[0] + idt;
-        double inv = rcp_full(bet);
-        double u = (idt * ph[0]) * inv;
+        double u, gg;
+        pivot(b[0] + idt, idt * ph[0], c[0], u, gg);
         ph[0] = u;
         for (int i = 1; i < L; i++) {
-            double gg = c[(i - 1) * S] * inv;
             gm[i * nt] = gg;
-            double ai = a[i * S];
-            bet = fma(-ai, gg, b[i * S] + idt);
-            inv = rcp_full(bet);
-            u = fma(-ai, u, idt * ph[i * tp]) * inv;
+            const double ai = a[i * S];
+            pivot(fma(-ai, gg, b[i * S] + idt), fma(-ai, u, idt * ph[i * tp]),
+                  i < L - 1 ? c[i * S] : 1.0, u, gg);
             ph[i * tp] = u;
         }
         for (int i = L - 2; i >= 0; i--) {
@@ -215,14 +212,13 @@ __global__ void k_tridiag_batch(const double *a, const double *b, const double *
         return;
     const double *as = a + s * n, *bs = b + s * n, *cs = c + s * n, *rs = r + s * n;
     double *us = u + s * n, *gs = gam + s * n;
-    double bet = bs[0];
-    double inv = rcp_full(bet);
-    us[0] = rs[0] * inv;
+    double x, g;
+    pivot(bs[0], rs[0], n > 1 ? cs[0] : 1.0, x, g);
+    us[0] = x;
     for (int j = 1; j < n; j++) {
-        gs[j] = cs[j - 1] * inv;
-        bet = fma(-as[j], gs[j], bs[j]);
-        inv = rcp_full(bet);
-        us[j] = fma(-as[j], us[j - 1], rs[j]) * inv;
+        gs[j] = g;
+        pivot(fma(-as[j], g, bs[j]), fma(-as[j], x, rs[j]), j < n - 1 ? cs[j] : 1.0, x, g);
+        us[j] = x;
     }
     for (int j = n - 2; j >= 0; j--)
         us[j] = fma(-gs[j + 1], us[j + 1], us[j]);

@@ -24,6 +24,44 @@ def test_refined_reciprocal(cuda_lib):
     assert (ulps == 0).mean() > 0.99
 
 
+def _pivot_inputs(kind, n):
+    rng = np.random.default_rng(7)
+    bits = lambda: rng.integers(0, 1 << 64, n, dtype=np.uint64).view(np.float64)
+    if kind == "any bits":  # every exponent, subnormals, infinities and NaN
+        return bits(), bits(), bits()
+    x = np.exp(rng.uniform(-80, 80, n))
+    t = rng.choice([-1.0, 1.0], n) * np.exp(rng.uniform(-600, 600, n))
+    c = -rng.uniform(0, 1, n)
+    if kind == "short mantissas":  # exact products, ties, mantissas next to 1 and 2
+        x = np.ldexp(1 + rng.integers(-64, 64, n) * 2.0 ** -52, rng.integers(-140, 140, n))
+        t = np.ldexp(1 + rng.integers(-64, 64, n) * 2.0 ** -rng.integers(5, 53, n),
+                     rng.integers(-1060, 1020, n))
+    if kind == "pivots":  # the sweeps' range, with the zero couplings of the boundary rows
+        x, t = 1 + np.exp(rng.uniform(-20, 8, n)), t ** 0.02
+        c[::7] = 0.0
+    return x, t, c
+
+
+@pytest.mark.parametrize("kind", ["pivots", "wide", "short mantissas", "any bits"])
+def test_integer_pivot_gives_the_bits_of_the_doubles(cuda_lib, kind):
+    """t * (1/x) and c * (1/x) on the integer pipes are, bit for bit, what the
+    FP64 instructions give (rounding, signs, and every value that leaves the
+    integers' range: zeros, subnormals, overflows, infinities; NaN as NaN)."""
+    import torch
+    from dadi_gb300 import _lib
+    n = 1 << 20
+    with np.errstate(all="ignore"):
+        xtc = np.concatenate(_pivot_inputs(kind, n))
+    d = torch.from_numpy(xtc).cuda()
+    o = torch.empty(4 * n, dtype=torch.float64, device="cuda")
+    _lib.check(cuda_lib.dgb_probe_pivot(_lib.dptr(d), _lib.dptr(o), n,
+                                        _lib.stream_handle(torch)), "pivot")
+    o = o.cpu().numpy()
+    got, want = o[:2 * n], o[2 * n:]
+    same = (got.view(np.int64) == want.view(np.int64)) | (np.isnan(got) & np.isnan(want))
+    assert same.all()
+
+
 def test_fp64_rate_and_idle_lanes(cuda_lib):
     """The FP64 FMA rate is positive and a warp instruction with a quarter of
     its lanes active takes as long as a full one (idle lanes are not free),
