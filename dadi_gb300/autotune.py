@@ -8,18 +8,14 @@ The knobs, each a real alternative the kernels implement:
   CTA per work item, each retiring after its item (what lets concurrent
   launches share SMs);
 * ... or "per_grid": one persistent launch per grid size, each shaped for
-  its own L (CTAs per SM, warps per CTA, two work items per CTA for a grid
-  of 73-128 points where that fills the lanes better), on side streams so
-  that one launch's tail overlaps the
-  next;
+  its own L (CTAs per SM, warps per CTA), on side streams so that one
+  launch's tail overlaps the next;
 * gam placement — the Thomas recurrence's scratch in shared memory (fewer
   CTAs per SM when the density already fills it) or in a per-CTA slice of
   the workspace (more CTAs per SM, L2 traffic on the back substitution);
-* threads per CTA — 0 lets the engine choose the fewest warps that hold
-  every line of the launch's largest grid (fuller warps: the FP64 pipe
-  charges a warp instruction whatever its active lanes), so per_grid runs
-  grids of up to 96 points on three warps; 128 forces four warps, the check
-  on that rule.
+* threads per CTA — 0 lets the engine run the factors of each sweep on other
+  warps than its solves where gam placement allows (2: yes, 1: no); 128 runs
+  both on four warps.
 
 `tune_batch2d` times every candidate on a sample of the batch — instances
 spread over the batch's cost distribution, so the sample has the batch's mix

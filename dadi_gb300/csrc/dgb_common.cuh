@@ -85,6 +85,8 @@ static __device__ __noinline__ double rcp_newton(double x)
 // = r0 2^21 (21 bits), -X rho mod 2^64 is the residual e = 1 - m r0 (|e| <
 // 2^-19) in units of 2^-73, exactly; then 1/m = r0 (1 + e + e^2) is built in
 // units of 2^-96 with an error below 2^-67, and rounded to 53 bits.
+static __device__ __noinline__ double mul_fp64(double x, double y) { return x * y; }
+
 struct Mant {
     unsigned h, l; // 2^64 / m rounded to 53 bits: the top bit of h is set
 };
@@ -146,14 +148,34 @@ __device__ __forceinline__ unsigned rcp_exps(double x)
     return 0x3fd00000u - ((unsigned)__double2hiint(x) & 0xfff00000u);
 }
 
+// The double of mantissa y and exps (as mul_mant takes them).
+__device__ __forceinline__ double mant_double(const Mant &y, unsigned exps)
+{
+    return __hiloint2double((int)((y.h >> 11) + 0x3ff00000u + exps),
+                            (int)__funnelshift_r(y.l, y.h, 11));
+}
+
 __device__ __forceinline__ double rcp_full(double x)
 {
     bool bad;
     const Mant y = rcp_mant(x, bad);
-    double r = __hiloint2double((int)((y.h >> 11) + 0x3ff00000u + rcp_exps(x)),
-                                (int)__funnelshift_r(y.l, y.h, 11));
+    double r = mant_double(y, rcp_exps(x));
     if (bad)
         r = rcp_newton(x);
+    return r;
+}
+
+// x * y rounded as IEEE multiplication rounds (y an unpacked double).
+__device__ __forceinline__ double mul_full(double x, double y)
+{
+    const unsigned yh = (unsigned)__double2hiint(y), yl = (unsigned)__double2loint(y);
+    Mant m;
+    m.h = __funnelshift_l(yl, (yh & 0xfffffu) | 0x100000u, 11);
+    m.l = yl << 11;
+    bool bad = (yh & 0x7fffffffu) - 0x37f00000u >= 0x10000000u;
+    double r = mul_mant(x, m, (yh & 0xfff00000u) - 0x40000000u, bad);
+    if (bad)
+        r = mul_fp64(x, y);
     return r;
 }
 

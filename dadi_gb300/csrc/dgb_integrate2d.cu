@@ -18,8 +18,11 @@
 // from host bounds on the rows, or count rows, scan, fill rows.
 // The batched integration is a persistent launch whose CTAs pull work items
 // longest-first from an atomic counter (one launch over all grids, or one
-// per grid size with a CTA shaped for it, two items per CTA where that fills
-// the warps better: k_integrate2d_pair), or one CTA per item.
+// per grid size with a CTA shaped for it), or one CTA per item.  Under the
+// default delta_j the factorisations of a sweep run on other warps than its
+// solves (k_integrate2d_ws); k_integrate2d, one warp for both, serves the delj
+// trick, an explicit CTA size or scratch placement, and callers without
+// workspace.
 //
 // Reference: the time loop of Integration.two_pops (dadi/Integration.py:
 // 340-386) with implicit_2Dx / implicit_2Dy (dadi/integration2D.c:19-160).
@@ -35,6 +38,7 @@ namespace dgb {
 constexpr int K2_THREADS = 128;
 constexpr int K2_MAXG = DGB_B2_MAXG;
 constexpr int K2_ROW = 11; // DGB_ROW_STRIDE(2)
+constexpr int K2_AUTO_ANY_L = -2; // dgb_settings.threads: as 0
 
 struct K2Args {
     int ngrids;
@@ -143,6 +147,44 @@ __device__ __forceinline__ void k2_axis_scalars(AxisScalars &s, int a, const dou
               s.bcs, s.bce);
 }
 
+// Work item wid of a launch.
+struct K2Item {
+    int wid, L, frozen, nomut, nsteps;
+    const double *xx, *src, *rows;
+    double *out;
+};
+
+__device__ __forceinline__ K2Item k2_item(const K2Args &A, int wid)
+{
+    K2Item I;
+    int sidx;
+    I.wid = wid;
+    if (A.items) {
+        // explicit item: its own grid, output slot (holding the initial
+        // density) and schedule
+        const dgb_item2d &it = A.items[wid];
+        I.L = it.L;
+        I.xx = A.xx_all + it.xx_off;
+        I.out = A.phi_out + it.out_off;
+        I.src = I.out;
+        sidx = (int)it.sched;
+        I.frozen = it.masks & 0xff;
+        I.nomut = it.masks >> 8 & 0xff;
+    } else {
+        const int inst = wid / A.ngrids, gi = wid - inst * A.ngrids;
+        I.L = A.L[gi];
+        I.xx = A.xx_all + A.xx_off[gi];
+        I.out = A.phi_out + A.out_off[gi] + (size_t)inst * I.L * I.L;
+        I.src = A.phi0_all ? A.phi0_all + A.phi0_off[gi] : I.out;
+        sidx = A.sched_per_grid ? wid : inst;
+        I.frozen = A.masks ? (A.masks[inst] & 0xff) : A.frozen_mask;
+        I.nomut = A.masks ? (A.masks[inst] >> 8 & 0xff) : A.nomut_mask;
+    }
+    I.rows = A.row_off ? A.table + A.row_off[sidx] * K2_ROW : A.table;
+    I.nsteps = A.row_off ? A.row_cnt[sidx] : A.fixed_cnt;
+    return I;
+}
+
 template <bool DELJ>
 __global__ void __launch_bounds__(K2_THREADS) k_integrate2d(K2Args A)
 {
@@ -168,34 +210,10 @@ __global__ void __launch_bounds__(K2_THREADS) k_integrate2d(K2Args A)
         if (w >= A.nwork)
             break;
         const int wid = A.order ? A.order[w] : w;
-        int inst, L, sidx, frozen, nomut;
-        const double *xx, *src;
-        double *out;
-        if (A.items) {
-            // explicit item: its own grid, output slot (holding the initial
-            // density) and schedule
-            const dgb_item2d &it = A.items[wid];
-            inst = wid;
-            L = it.L;
-            xx = A.xx_all + it.xx_off;
-            out = A.phi_out + it.out_off;
-            src = out;
-            sidx = (int)it.sched;
-            frozen = it.masks & 0xff;
-            nomut = it.masks >> 8 & 0xff;
-        } else {
-            inst = wid / A.ngrids;
-            const int gi = wid - inst * A.ngrids;
-            L = A.L[gi];
-            xx = A.xx_all + A.xx_off[gi];
-            out = A.phi_out + A.out_off[gi] + (size_t)inst * L * L;
-            src = A.phi0_all ? A.phi0_all + A.phi0_off[gi] : out;
-            sidx = A.sched_per_grid ? wid : inst;
-            frozen = A.masks ? (A.masks[inst] & 0xff) : A.frozen_mask;
-            nomut = A.masks ? (A.masks[inst] >> 8 & 0xff) : A.nomut_mask;
-        }
-        const double *rows = A.row_off ? A.table + A.row_off[sidx] * K2_ROW : A.table;
-        const int nsteps = A.row_off ? A.row_cnt[sidx] : A.fixed_cnt;
+        const K2Item I = k2_item(A, wid);
+        const int L = I.L, frozen = I.frozen, nomut = I.nomut, nsteps = I.nsteps;
+        const double *xx = I.xx, *src = I.src, *rows = I.rows;
+        double *out = I.out;
 
         // grid constants and initial density
         for (int i = tid; i < L; i += blockDim.x) {
@@ -302,203 +320,329 @@ __global__ void __launch_bounds__(K2_THREADS) k_integrate2d(K2Args A)
     }
 }
 
-// ------------------------------------------------ two items per CTA
+// ------------------------------------- factors and solves on their own warps
 
-// k_integrate2d for a launch over one grid of L points with two work items
-// per CTA, stepped together: the 2L lines of a sweep (L of each item) are
-// spread over ceil(2L/32) warps, so a grid whose L lines would leave a
-// fourth warp mostly empty (L = 100: 25 of 32 lanes busy on four warps)
-// fills its warps better (200 lines on seven warps: 29 of 32).  Each item
-// keeps its own density, schedule, masks and coefficient vectors; the grid
-// constants are shared.  The two items are neighbours in the longest-first
-// order, so their step counts are close; the shorter one's lanes idle for
-// the difference.  Per line the arithmetic is k_integrate2d's (default
-// delta_j only), so the results are bitwise the same.  Thomas scratch: a 2L x L slice of the
-// workspace per CTA (element p of line q at gam[p*2L + q]).
-constexpr int K2P_MAXTHREADS = 256;
-// dgb_settings.threads value: two work items per CTA at any grid size where
-// that fills the warps better (the automatic choice keeps it to L > 96)
-constexpr int K2_PAIR_ANY_L = -2;
+// k_integrate2d with each sweep's factorisation on other warps than its
+// solves.  Of a line's Thomas recurrence only t = phi - a u, u = t inv and
+// the back substitution need the density; the pivots, their reciprocals inv
+// and the couplings g = c inv follow from the parameter row alone.  So while
+// the solve warps (one line per lane) run a sweep, as many factor warps form
+// a, inv and g of the next one and hand them over through the workspace (one
+// set per axis, in L2), with one barrier per sweep.  Per grid point the chain
+// of the solve is a fused multiply-add, a product on the integer pipes and a
+// back substitution, and the chain of the factors a fused multiply-add, a
+// reciprocal and a product, where the fused sweep's warps run one after the
+// other.  The arithmetic per line is solve_line's, so the results are bitwise
+// the same.  Measured, microseconds per step with one warp for both / with
+// this kernel: one grid alone, L = 31 25 / 14, 64 45 / 25, 100 69 / 45, 128
+// 83 / 56, 133 (two rounds of lines on four warps / five warps) 168 / 72; 8
+// grids per SM, per grid and SM, L = 45 18.6 / 11.6, 80 30 / 24, 90 38 / 30,
+// 100 42 / 43, 133 169 / 81.
+constexpr int K2W_MAXWARPS = 5; // of lines
+constexpr int K2W_STEPS = 16;   // steps whose scalars are formed at once
 
-struct K2PairShared {
-    AxisScalars ax[2][2]; // [item slot][axis]
-    double inj[2];
-    int item[2];
+struct K2WShared {
+    AxisScalars ax[2 * K2W_STEPS][2]; // ring over the steps
+    double inj[2 * K2W_STEPS];
+    int item;
 };
 
-__host__ __device__ inline size_t k2_pair_doubles(int L)
+// Workspace of one CTA: [axis][inv, g, a][row][line] (keep_a), lines padded to
+// 128 bytes.
+__host__ __device__ inline int k2w_pitch(int L) { return (L + 15) / 16 * 16; }
+
+__host__ __device__ inline size_t k2w_slice_doubles(int L, bool keep_a)
 {
-    return 2 * (size_t)L * odd_pitch(L) + 6 * (size_t)L + 4 * 5 * (size_t)L;
+    return (size_t)(keep_a ? 6 : 4) * L * k2w_pitch(L);
 }
 
-// Coefficient vectors of (slot, axis) index sa = 2*slot + axis.
-__device__ __forceinline__ AxisVecs k2p_vecs(double *vbase, int sa, int L)
+__host__ __device__ inline size_t k2w_smem_doubles(int L)
 {
-    double *p = vbase + (size_t)sa * 5 * L;
-    AxisVecs v;
-    v.A1 = p;
-    v.A0 = p + L;
-    v.C1 = p + 2 * L;
-    v.C0 = p + 3 * L;
-    v.B0 = p + 4 * L;
-    v.G = v.Pv = v.Qv = v.VI = v.DF = nullptr;
-    return v;
+    return (size_t)L * odd_pitch(L) + 6 * (size_t)L + 10 * (size_t)L;
 }
 
-__global__ void __launch_bounds__(K2P_MAXTHREADS, 1) k_integrate2d_pair(K2Args A)
+__device__ __forceinline__ void bar_group(int id, int n)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
+// 1/bet and c * (1/bet).
+__device__ __forceinline__ void pivot_inv(double bet, double c, double &inv, double &g)
+{
+    bool bad;
+    const Mant y = rcp_mant(bet, bad);
+    const unsigned exps = rcp_exps(bet);
+    g = mul_mant(c, y, exps, bad);
+    inv = mant_double(y, exps);
+    if (bad) {
+        inv = rcp_newton(bet);
+        g = mul_fp64(c, inv);
+    }
+}
+
+// The factors of one line: f[0][i] = 1/bet_i, f[1][i] = g_i and, where KEEP_A,
+// f[2][i] = a_i; array k at f + k * stride, row i at i * LP.
+template <bool KEEP_A>
+__device__ __forceinline__ void k2w_factor(const AxisVecs &v, const AxisScalars &s, int L,
+                                           double W, double bs, double be, double *f,
+                                           size_t stride, int LP)
+{
+    double *fi = f, *fg = f + stride, *fa = f + 2 * stride;
+    double inv, g;
+    pivot_inv(fma(W, s.B1s, v.B0[0]) + bs, fma(W, v.C1[0], v.C0[0]), inv, g);
+    fi[0] = inv;
+    fg[0] = g;
+    double a = fma(W, v.A1[1], v.A0[1]), c = fma(W, v.C1[1], v.C0[1]), b0 = v.B0[1];
+    for (int i = 1; i < L - 1; i++) {
+        const double bet = fma(-a, g, b0), ai = a, ci = c;
+        a = fma(W, v.A1[i + 1], v.A0[i + 1]);
+        c = fma(W, v.C1[i + 1], v.C0[i + 1]);
+        b0 = v.B0[i + 1];
+        pivot_inv(bet, ci, inv, g);
+        if (KEEP_A)
+            fa[i * LP] = ai;
+        fi[i * LP] = inv;
+        fg[i * LP] = g;
+    }
+    if (KEEP_A)
+        fa[(L - 1) * LP] = a;
+    fi[(L - 1) * LP] = rcp_full(fma(-a, g, fma(W, s.B1e, b0) + be));
+}
+
+// The solve of one line from its factors (as k2w_factor leaves them); element
+// p at ph[p * sp].  The factors of the next rows are loaded ahead of the rows
+// that use them.
+template <bool KEEP_A>
+__device__ __forceinline__ void k2w_solve(double *__restrict__ ph, int sp, int L,
+                                          const AxisVecs &v, double W,
+                                          const double *__restrict__ f, size_t stride, int LP)
+{
+    constexpr int B = 4, C = 8;
+    const double *fi = f, *fg = f + stride, *fa = f + 2 * stride;
+    double av[B], iv[B], gv[C];
+#pragma unroll
+    for (int k = 0; k < B; k++) {
+        const int r = min(1 + k, L - 1);
+        iv[k] = __ldcg(fi + r * LP);
+        if (KEEP_A)
+            av[k] = __ldcg(fa + r * LP);
+    }
+    double u = mul_full(ph[0], __ldcg(fi));
+    ph[0] = u;
+    int i = 1;
+    for (; i + B <= L; i += B) {
+        double an[B], in[B], pv[B];
+#pragma unroll
+        for (int k = 0; k < B; k++) {
+            const int r = min(i + B + k, L - 1);
+            in[k] = __ldcg(fi + r * LP);
+            if (KEEP_A)
+                an[k] = __ldcg(fa + r * LP);
+            else
+                av[k] = fma(W, v.A1[i + k], v.A0[i + k]);
+            pv[k] = ph[(i + k) * sp];
+        }
+#pragma unroll
+        for (int k = 0; k < B; k++) {
+            u = mul_full(fma(-av[k], u, pv[k]), iv[k]);
+            ph[(i + k) * sp] = u;
+        }
+#pragma unroll
+        for (int k = 0; k < B; k++) {
+            if (KEEP_A)
+                av[k] = an[k];
+            iv[k] = in[k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < C; k++)
+        gv[k] = __ldcg(fg + max(L - 2 - k, 0) * LP);
+#pragma unroll
+    for (int k = 0; k < B - 1; k++)
+        if (i + k < L) {
+            const double a = KEEP_A ? av[k] : fma(W, v.A1[i + k], v.A0[i + k]);
+            u = mul_full(fma(-a, u, ph[(i + k) * sp]), iv[k]);
+            ph[(i + k) * sp] = u;
+        }
+    i = L - 2;
+    for (; i >= C - 1; i -= C) {
+        double gn[C], pv[C];
+#pragma unroll
+        for (int k = 0; k < C; k++) {
+            gn[k] = __ldcg(fg + max(i - C - k, 0) * LP);
+            pv[k] = ph[(i - k) * sp];
+        }
+#pragma unroll
+        for (int k = 0; k < C; k++) {
+            u = fma(-gv[k], u, pv[k]);
+            ph[(i - k) * sp] = u;
+        }
+#pragma unroll
+        for (int k = 0; k < C; k++)
+            gv[k] = gn[k];
+    }
+#pragma unroll
+    for (int k = 0; k < C - 1; k++)
+        if (i - k >= 0) {
+            u = fma(-gv[k], u, ph[(i - k) * sp]);
+            ph[(i - k) * sp] = u;
+        }
+}
+
+// Groups of W warps of a CTA: solves, factors, and (few lines, where the
+// vectors would hold up the solves) the vectors.
+__host__ __device__ constexpr int k2w_groups(int W) { return W <= 2 ? 3 : 2; }
+
+template <int W, bool KEEP_A>
+__global__ void __launch_bounds__(32 * W * k2w_groups(W), W == 1 ? 5 : W == 2 ? 3 : 2)
+    k_integrate2d_ws(K2Args A)
 {
     extern __shared__ __align__(16) double smem[];
-    __shared__ K2PairShared S;
+    __shared__ K2WShared S;
+    constexpr int ng = 32 * W; // threads of a group
     const int tid = threadIdx.x;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int nwarps = blockDim.x >> 5;
-    const int L = A.L[0];
-    const int pitch = odd_pitch(L);
-    const size_t psz = (size_t)L * pitch;
-    double *phi0 = smem; // slot s at phi0 + s * psz
+    constexpr bool P = k2w_groups(W) == 3;
+    static_assert(KEEP_A || !P, "a third group rebuilds the vectors that the solves would read");
+    const int group = tid / ng, q = tid - group * ng;
+    const int pitch = odd_pitch(A.Lmax);
+    double *phi = smem;
     GridVecs g;
-    double *p = smem + 2 * psz;
-    g.x = p; p += L;
-    g.xv = p; p += L;
-    g.dfac = p; p += L;
-    g.xInt = p; p += L;
-    g.ih = p; p += L;
-    g.dx = p; p += L;
-    double *vbase = p; // 4 x 5 x L doubles
-    double *gam = A.gam_glob + (size_t)blockIdx.x * 2 * L * L;
-    const double *xx = A.xx_all + A.xx_off[0];
+    double *p = smem + (size_t)A.Lmax * pitch;
+    g.x = p; p += A.Lmax;
+    g.xv = p; p += A.Lmax;
+    g.dfac = p; p += A.Lmax;
+    g.xInt = p; p += A.Lmax;
+    g.ih = p; p += A.Lmax;
+    g.dx = p; p += A.Lmax;
+    auto vecs = [&](int a) {
+        double *w = p + (size_t)a * 5 * A.Lmax;
+        AxisVecs v;
+        v.A1 = w;
+        v.A0 = w + A.Lmax;
+        v.C1 = w + 2 * A.Lmax;
+        v.C0 = w + 3 * A.Lmax;
+        v.B0 = w + 4 * A.Lmax;
+        v.G = v.Pv = v.Qv = v.VI = v.DF = nullptr;
+        return v;
+    };
+    double *slice = A.gam_glob + (size_t)blockIdx.x * k2w_slice_doubles(A.Lmax, KEEP_A);
 
-    // grid constants, once for every item of the launch
-    for (int i = tid; i < L; i += blockDim.x) {
-        double x = xx[i];
-        g.x[i] = x;
-        g.xv[i] = x * (1. - x);
-        if (i < L - 1) {
-            double d = xx[i + 1] - x;
-            g.dx[i] = d;
-            g.ih[i] = 1.0 / (2 * d);
-            g.xInt[i] = 0.5 * (xx[i + 1] + x);
-        }
-    }
-    __syncthreads();
-    for (int i = tid; i < L; i += blockDim.x) {
-        if (i == 0)
-            g.dfac[i] = 2. / g.dx[0];
-        else if (i == L - 1)
-            g.dfac[i] = 2. / g.dx[L - 2];
-        else
-            g.dfac[i] = 2. / (g.dx[i] + g.dx[i - 1]);
-    }
-    __syncthreads();
-    const int j0 = (g.x[0] == 0.0) ? 0 : -1;
-    const int j1 = (g.x[L - 1] == 1.0) ? L - 1 : -1;
-
-    // S.item is written by thread 0 and read by all between the barrier that
-    // follows the write and the next barrier thread 0 must pass to write again.
     for (int iter = 0;; iter++) {
-        if (tid == 0) {
-            const int base =
-                A.counter ? atomicAdd(A.counter, 2) : (iter == 0 ? 2 * (int)blockIdx.x : A.nwork);
-            S.item[0] = base;
-            S.item[1] = base + 1;
-        }
+        if (tid == 0)
+            S.item = A.counter ? atomicAdd(A.counter, 1) : (iter == 0 ? (int)blockIdx.x : A.nwork);
         __syncthreads();
-        if (S.item[0] >= A.nwork)
+        const int w = S.item;
+        if (w >= A.nwork)
             break;
-        const int ns = (S.item[1] < A.nwork) ? 2 : 1; // item slots in use
-        int nst0 = 0, nst1 = 0, fr0 = 0, fr1 = 0, nm0 = 0, nm1 = 0;
-        const double *rows0 = nullptr, *rows1 = nullptr;
-        double *out0 = nullptr, *out1 = nullptr;
-        for (int s = 0; s < ns; s++) {
-            const int wid = A.order ? A.order[S.item[s]] : S.item[s];
-            double *out = A.phi_out + A.out_off[0] + (size_t)wid * L * L;
-            const double *src = A.phi0_all ? A.phi0_all + A.phi0_off[0] : out;
-            const int fr = A.masks ? (A.masks[wid] & 0xff) : A.frozen_mask;
-            const int nm = A.masks ? (A.masks[wid] >> 8 & 0xff) : A.nomut_mask;
-            const double *rows = A.row_off ? A.table + A.row_off[wid] * K2_ROW : A.table;
-            const int nst = A.row_off ? A.row_cnt[wid] : A.fixed_cnt;
-            if (s == 0) {
-                out0 = out; fr0 = fr; nm0 = nm; rows0 = rows; nst0 = nst;
-            } else {
-                out1 = out; fr1 = fr; nm1 = nm; rows1 = rows; nst1 = nst;
+        const K2Item I = k2_item(A, A.order ? A.order[w] : w);
+        const int L = I.L, LP = k2w_pitch(L);
+        const size_t stride = (size_t)L * LP;
+        for (int i = tid; i < L; i += blockDim.x) {
+            double x = I.xx[i];
+            g.x[i] = x;
+            g.xv[i] = x * (1. - x);
+            if (i < L - 1) {
+                double d = I.xx[i + 1] - x;
+                g.dx[i] = d;
+                g.ih[i] = 1.0 / (2 * d);
+                g.xInt[i] = 0.5 * (I.xx[i + 1] + x);
             }
-            double *ph = phi0 + s * psz;
-            for (int idx = tid; idx < L * L; idx += blockDim.x) {
-                int r = idx / L, c = idx - r * L;
-                ph[r * pitch + c] = src[idx];
-            }
+        }
+        for (int idx = tid; idx < L * L; idx += blockDim.x) {
+            int r = idx / L, c = idx - r * L;
+            phi[r * pitch + c] = I.src[idx];
         }
         __syncthreads();
-        const int nmax = max(nst0, nst1);
-        const int nl = ns * L; // lines of one sweep over the slots in use
-        const int lpw = (nl + nwarps - 1) / nwarps;
-
-        for (int step = 0; step < nmax; step++) {
-            const bool act0 = step < nst0, act1 = step < nst1;
-            // ---- step scalars: lane 2s+a of warp 0 for (slot s, axis a),
-            // lane 4+s the injection of slot s
-            if (warp == 0 && lane < 6) {
-                const int s = (lane < 4) ? (lane >> 1) : lane - 4;
-                if (s ? act1 : act0) {
-                    const double *row = (s ? rows1 : rows0) + (size_t)step * K2_ROW;
-                    if (lane < 4)
-                        k2_axis_scalars(S.ax[s][lane & 1], lane & 1, row, g, L);
-                    else
-                        S.inj[s] = inject_value(2, row[0], row[1], g.x[0], g.x[1], g.x[2]);
-                }
-            }
-            __syncthreads();
-            // ---- per-axis vectors of both slots and mutation injection
-            for (int t = tid; t < ns * 2 * L; t += blockDim.x) {
-                const int sa = t / L, i = t - sa * L; // sa = 2*slot + axis
-                if ((sa >> 1) ? act1 : act0) {
-                    AxisVecs v = k2p_vecs(vbase, sa, L);
-                    build_axis_entry(i, L, g, S.ax[sa >> 1][sa & 1], 1.0, false, v);
-                }
-            }
-            if (tid == 0) {
-                for (int s = 0; s < ns; s++) {
-                    if (!(s ? act1 : act0))
-                        continue;
-                    const int fr = s ? fr1 : fr0, nm = s ? nm1 : nm0;
-                    double *ph = phi0 + s * psz;
-                    if (!(fr & 1) && !(nm & 1))
-                        ph[1 * pitch + 0] += S.inj[s];
-                    if (!(fr & 2) && !(nm & 2))
-                        ph[0 * pitch + 1] += S.inj[s];
-                }
-            }
-            __syncthreads();
-            // ---- x sweep (axis 0) then y sweep (axis 1) over both slots' lines
-            for (int a = 0; a < 2; a++) {
-                const int sp = (a == 0) ? pitch : 1;
-                const int sl = (a == 0) ? 1 : pitch;
-                for (int k = lane; k < lpw; k += 32) {
-                    const int q = warp * lpw + k;
-                    if (q >= nl)
-                        break;
-                    const int s = (q >= L) ? 1 : 0;
-                    const int line = q - s * L;
-                    if (!(s ? act1 : act0) || ((s ? fr1 : fr0) & (1 << a)))
-                        continue;
-                    const AxisScalars &sc = S.ax[s][a];
-                    const AxisVecs v = k2p_vecs(vbase, 2 * s + a, L);
-                    const double W = sc.mig[1 - a] * g.x[line];
-                    const double bs = (line == j0) ? sc.bcs : 0.0;
-                    const double be = (line == j1) ? sc.bce : 0.0;
-                    double *ph = phi0 + s * psz + (size_t)line * sl;
-                    solve_line(ph, sp, gam + q, 2 * L, L, W, bs, be, v, sc);
-                }
-                __syncthreads();
-            }
+        for (int i = tid; i < L; i += blockDim.x) {
+            if (i == 0)
+                g.dfac[i] = 2. / g.dx[0];
+            else if (i == L - 1)
+                g.dfac[i] = 2. / g.dx[L - 2];
+            else
+                g.dfac[i] = 2. / (g.dx[i] + g.dx[i - 1]);
         }
-        for (int s = 0; s < ns; s++) {
-            const double *ph = phi0 + s * psz;
-            double *out = s ? out1 : out0;
-            for (int idx = tid; idx < L * L; idx += blockDim.x) {
-                int r = idx / L, c = idx - r * L;
-                out[idx] = ph[r * pitch + c];
+        __syncthreads();
+        const int j0 = (g.x[0] == 0.0) ? 0 : -1;
+        const int j1 = (g.x[L - 1] == 1.0) ? L - 1 : -1;
+        const int nsw = 2 * I.nsteps; // sweep m: axis m & 1 of step m >> 1
+
+        // Phase m: the solve warps run sweep m and then form the vectors of
+        // sweep m + 2 (the same axis; the scalars of K2W_STEPS steps when
+        // they run out); the factor warps run sweep m + 1.
+        auto prepare = [&](int m) {
+            const int a = m & 1, n = m >> 1;
+            if (m >= nsw)
+                return;
+            if (a == 0 && n % K2W_STEPS == 0) {
+                const int st = n + (q >> 1);
+                const double *row = I.rows + (size_t)st * K2_ROW;
+                if (q < 2 * K2W_STEPS && st < I.nsteps)
+                    k2_axis_scalars(S.ax[st % (2 * K2W_STEPS)][q & 1], q & 1, row, g, L);
+                if (q < 2 * K2W_STEPS && st < I.nsteps && !(q & 1))
+                    S.inj[st % (2 * K2W_STEPS)] =
+                        inject_value(2, row[0], row[1], g.x[0], g.x[1], g.x[2]);
+                bar_group(2, ng);
             }
+            if (I.frozen >> a & 1)
+                return;
+            AxisVecs v = vecs(a);
+            for (int i = q; i < L; i += ng)
+                build_axis_entry(i, L, g, S.ax[n % (2 * K2W_STEPS)][a], 1.0, false, v);
+        };
+        const bool prep = group == (P ? 2 : 0);
+        if (prep) {
+            prepare(0);
+            prepare(1);
+        }
+        __syncthreads();
+        for (int m = -1; m < nsw; m++) {
+            if (group == 1) {
+                const int a = (m + 1) & 1;
+                if (m + 1 < nsw && !(I.frozen >> a & 1) && q < L) {
+                    const AxisScalars &s = S.ax[(m + 1) / 2 % (2 * K2W_STEPS)][a];
+                    k2w_factor<KEEP_A>(vecs(a), s, L, s.mig[1 - a] * g.x[q],
+                                       (q == j0) ? s.bcs : 0.0, (q == j1) ? s.bce : 0.0,
+                                       slice + a * (KEEP_A ? 3 : 2) * stride + q, stride, LP);
+                }
+            } else if (P && group == 2) {
+                prepare(m + 2);
+            } else if (m >= 0) {
+                const int a = m & 1, k = m >> 1;
+                if (a == 0) {
+                    if (A.ckpt && k % A.ckpt_every == 0) {
+                        // checkpoint for the adjoint: phi before this step, row-major
+                        double *c = A.ckpt + A.ckpt_off[I.wid] + (size_t)(k / A.ckpt_every) * L * L;
+                        for (int idx = q; idx < L * L; idx += ng) {
+                            int r = idx / L, cc = idx - r * L;
+                            c[idx] = phi[r * pitch + cc];
+                        }
+                        bar_group(1, ng);
+                    }
+                    if (q == 0) {
+                        const double inj = S.inj[k % (2 * K2W_STEPS)];
+                        if (!(I.frozen & 1) && !(I.nomut & 1))
+                            phi[1 * pitch + 0] += inj;
+                        if (!(I.frozen & 2) && !(I.nomut & 2))
+                            phi[0 * pitch + 1] += inj;
+                    }
+                    bar_group(1, ng);
+                }
+                if (!(I.frozen >> a & 1) && q < L)
+                    k2w_solve<KEEP_A>(phi + (size_t)q * ((a == 0) ? 1 : pitch),
+                                      (a == 0) ? pitch : 1, L, vecs(a),
+                                      S.ax[k % (2 * K2W_STEPS)][a].mig[1 - a] * g.x[q],
+                                      slice + a * (KEEP_A ? 3 : 2) * stride + q, stride, LP);
+                if (!P) {
+                    if (!KEEP_A)
+                        bar_group(1, ng); // the solves still read the axis's vectors
+                    prepare(m + 2);
+                }
+            }
+            __syncthreads();
+        }
+        for (int idx = tid; idx < L * L; idx += blockDim.x) {
+            int r = idx / L, c = idx - r * L;
+            I.out[idx] = phi[r * pitch + c];
         }
         __syncthreads();
     }
@@ -726,39 +870,6 @@ static int k2_occupancy(bool delj, size_t smem, int threads = K2_THREADS)
     return nb > 0 ? nb : 1;
 }
 
-// Resident two-item CTAs per SM (k_integrate2d_pair), as k2_occupancy.
-static int k2_pair_occupancy(size_t smem, int threads)
-{
-    int nb = 0;
-    raise_smem_limit(k_integrate2d_pair);
-    cudaError_t e =
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_integrate2d_pair, threads, smem);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return nb;
-}
-
-// Threads of a two-item CTA for grids of L points when pairing pays: one
-// grid of 97-128 points (a single item needs four warps there) whose 2L
-// lines fill their warps at least 5 % better than L lines fill four; else 0.
-// Threads of a two-item CTA for grids of L points, or 0 where one item per
-// CTA is kept: pairs only when they fill the warps' lanes at least 5 points
-// better, and (unless any_L) only for L > 72.  Measured on the 4096-instance
-// IM batch: at L = 100 (200 lines on 7 warps against 100 on 4) the launch
-// went from 4977 to 4590 ms, at L = 80 (160 lines on 5 warps against 80 on
-// 3, one CTA per SM instead of three) the step's integration from 11.30 to
-// 11.00 s; at L = 90 pairs fill the lanes no better (180 of 192).
-static int k2_pair_threads(int L, bool any_L = false)
-{
-    if ((!any_L && L <= 72) || L > K2P_MAXTHREADS / 2)
-        return 0;
-    const int w1 = (L + 31) / 32, w2 = (2 * L + 31) / 32;
-    const double f1 = (double)L / (32 * w1), f2 = (double)(2 * L) / (32 * w2);
-    return (f2 >= f1 + 0.05) ? 32 * w2 : 0;
-}
-
 static int k2_num_sms()
 {
     int dev = 0, nsm = 0;
@@ -781,7 +892,7 @@ static int k2_num_sms()
 static int k2_pick_threads(const dgb_settings *settings, bool delj, size_t smem, int Lmax,
                            int &occ)
 {
-    const int want = (settings->threads == K2_PAIR_ANY_L) ? 0 : settings->threads;
+    const int want = (settings->threads == K2_AUTO_ANY_L) ? 0 : settings->threads;
     if (want != 0 && want != 64 && want != 96 && want != 128)
         return 0;
     int warps = std::min(4, std::max(2, (Lmax + 31) / 32));
@@ -789,6 +900,83 @@ static int k2_pick_threads(const dgb_settings *settings, bool delj, size_t smem,
         warps = want / 32;
     occ = k2_occupancy(delj, smem + sizeof(K2Shared), 32 * warps);
     return 32 * warps;
+}
+
+template <int W> static void (*k2w_kernel(bool keep_a))(K2Args)
+{
+    // (with a third group the vectors of an axis are rebuilt beside its
+    // solves, which then take a from the workspace)
+    return keep_a || k2w_groups(W) == 3 ? k_integrate2d_ws<W, true>
+                                        : k_integrate2d_ws<W, k2w_groups(W) == 3>;
+}
+
+// Whether the caller leaves the shape of a batched launch to the rules here.
+static bool k2w_auto(const dgb_settings *s)
+{
+    return (s->threads == 0 || s->threads == K2_AUTO_ANY_L) && s->gam_placement != 1;
+}
+
+// CTAs of k_integrate2d_ws per SM for nwork items on sms SMs.  One CTA uses
+// half to three quarters of the FP64 pipe (an SM's cycles per grid point and
+// warp of lines, one CTA / as many as fit: L = 45 220 / 98, 64 181 / 99, 80
+// 136 / 95, 90 151 / 108, 100 110 / 103), but a second one slows the first,
+// and a batch of few items per SM ends when its longest item does: 257 IM sets
+// on three grids of 31-45 points (5 items per SM) took 88 ms with one CTA and
+// 101 with two, 1000 sets at pts 80/90/100 652 with one and 519 with two.
+static int k2w_per_sm(long nwork, int sms)
+{
+    return (int)std::max<long>(1, std::min<long>(5, nwork / (3L * sms)));
+}
+
+// Launch k_integrate2d_ws over A's work (queue counter already cleared, or
+// null: one item per CTA) on `sms` SMs with slices from `slices` on; -1 where
+// it does not apply: the delj trick, grids beyond five warps of lines or
+// shared memory, or too little workspace.  The solves take a from the
+// workspace where the slices of all CTAs stay within the L2 cache, and form it
+// again (one more FP64 instruction a point, a third less traffic) where not:
+// 152 grids of 128 points 90 us a step with a, 62 without; of 100 points 46
+// and 51.
+static int k2w_launch(K2Args &A, void *slices, size_t bytes, int sms, cudaStream_t st)
+{
+    const int warps = (A.Lmax + 31) / 32;
+    if (A.use_delj || warps > K2W_MAXWARPS)
+        return -1;
+    const int threads = 32 * warps * k2w_groups(warps);
+    const size_t smem = k2w_smem_doubles(A.Lmax) * sizeof(double);
+    int dev = 0, optin = 0, occ = 0, l2 = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
+            cudaSuccess ||
+        cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
+        return -1;
+    if (smem + sizeof(K2WShared) + 1024 > (size_t)optin)
+        return -1;
+    void (*(*const kernels[])(bool))(K2Args) = {k2w_kernel<1>, k2w_kernel<2>, k2w_kernel<3>,
+                                                k2w_kernel<4>, k2w_kernel<5>};
+    void (*kernel)(K2Args) = nullptr;
+    long nblocks = 0;
+    for (int keep = 1; keep >= (k2w_groups(warps) == 3 ? 1 : 0); keep--) {
+        const size_t slice = k2w_slice_doubles(A.Lmax, keep) * sizeof(double);
+        kernel = kernels[warps - 1](keep);
+        if (raise_smem_limit(kernel))
+            return -1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) !=
+            cudaSuccess) {
+            cudaGetLastError();
+            return -1;
+        }
+        const long want = std::min<long>((long)sms * std::min(occ, k2w_per_sm(A.nwork, sms)),
+                                         A.nwork);
+        nblocks = std::min<long>((long)(bytes / slice), want);
+        if (nblocks == want && (size_t)nblocks * slice <= (size_t)l2 / 10 * 8)
+            break;
+    }
+    if (nblocks < std::min(sms, A.nwork))
+        return -1;
+    A.gam_smem = 0;
+    A.gam_glob = (double *)slices;
+    kernel<<<(unsigned)nblocks, threads, smem, st>>>(A);
+    return cudaGetLastError() == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
 }
 
 int k2_integrate_table(double *phi, int L, const double *xx, const double *table, int nsteps,
@@ -809,6 +997,11 @@ int k2_integrate_table(double *phi, int L, const double *xx, const double *table
     A.Lmax = L;
     A.use_delj = use_delj;
     size_t bytes;
+    if (ws) {
+        const int rc = k2w_launch(A, ws, ws_bytes, 1, st);
+        if (rc != -1)
+            return rc;
+    }
     A.gam_smem = k2_smem_fits(L, true, use_delj, &bytes);
     if (!A.gam_smem) {
         if (!k2_smem_fits(L, false, use_delj, &bytes))
@@ -820,12 +1013,16 @@ int k2_integrate_table(double *phi, int L, const double *xx, const double *table
     return k2_launch(A, 1, bytes, st);
 }
 
-size_t k2_table_ws_bytes(int L) { return (size_t)L * L * sizeof(double); }
+size_t k2_table_ws_bytes(int L) { return k2w_slice_doubles(L, true) * sizeof(double); }
 
 size_t k2_batch_ws_bytes(int Lmax, long nwork)
 {
-    (void)nwork;
-    return 256 + (size_t)k2_num_sms() * 4 * Lmax * Lmax * sizeof(double);
+    const int sms = k2_num_sms();
+    const size_t scratch = (size_t)sms * 4 * Lmax * Lmax; // k_integrate2d, up to four CTAs per SM
+    const int per_sm = std::min(k2w_per_sm(nwork, sms), Lmax <= 64 ? 5 : 2);
+    const size_t slices = k2w_slice_doubles(Lmax, true) *
+                          (size_t)std::min<long>((long)sms * per_sm, std::max<long>(nwork, 1));
+    return 256 + std::max(scratch, slices) * sizeof(double);
 }
 
 // norder: integrate only the work items order[0 .. norder) (<= 0: all);
@@ -914,35 +1111,14 @@ int k2_batch(int ninst, const int *masks, const int *Ls, int ngrids, const doubl
     }
     if (threads == 0)
         return DGB_ERR_ARG;
-    // two work items per CTA where that fills the warps better (one grid,
-    // automatic thread count, no checkpoints, scratch in the workspace; the
-    // two-item kernel implements the default delta_j only, so the delj
-    // trick keeps one item per CTA)
-    const bool any_L = settings->threads == K2_PAIR_ANY_L;
-    const int pthreads = (ngrids == 1 && !ckpt && !use_s && (settings->threads == 0 || any_L) &&
-                          !A.use_delj)
-                             ? k2_pair_threads(Lmax, any_L)
-                             : 0;
-    if (pthreads) {
-        const size_t pbytes = k2_pair_doubles(Lmax) * sizeof(double);
-        int dev = 0, optin = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
-                cudaSuccess)
+    // automatic shape: factors and solves on their own warps
+    if (k2w_auto(settings)) {
+        if (cudaMemsetAsync(A.counter, 0, sizeof(int), st) != cudaSuccess)
             return DGB_ERR_CUDA;
-        const int pocc = (pbytes + sizeof(K2PairShared) + 1024 <= (size_t)optin)
-                             ? k2_pair_occupancy(pbytes, pthreads)
-                             : 0;
-        long pblocks = std::min<long>((long)((ws_bytes - 256) / (2 * slice)), (long)nsm * pocc);
-        pblocks = std::min<long>(pblocks, (A.nwork + 1) / 2);
-        if (pblocks >= 1) {
-            A.gam_smem = 0;
-            A.gam_glob = (double *)((char *)ws + 256);
-            if (cudaMemsetAsync(A.counter, 0, sizeof(int), st) != cudaSuccess)
-                return DGB_ERR_CUDA;
-            k_integrate2d_pair<<<(unsigned)pblocks, pthreads, pbytes, st>>>(A);
-            return cudaGetLastError() == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
-        }
+        const int rc = k2w_launch(A, (char *)ws + 256, ws_bytes - 256,
+                                  reserve_sms > 0 ? std::max(1, nsm - reserve_sms) : nsm, st);
+        if (rc != -1)
+            return rc;
     }
     if (nblocks < 1)
         return DGB_ERR_WORKSPACE;
@@ -1157,6 +1333,14 @@ extern "C" int dgb_items2d_integrate(const dgb_item2d *items, int nitems, int Lm
     const int threads = k2_pick_threads(settings, A.use_delj, smem, Lmax, occ);
     if (threads == 0)
         return DGB_ERR_ARG;
+    if (!one_per_cta && k2w_auto(settings)) {
+        if (cudaMemsetAsync(A.counter, 0, sizeof(int), (cudaStream_t)stream) != cudaSuccess)
+            return DGB_ERR_CUDA;
+        const int rc = k2w_launch(A, (char *)ws + 256, ws_bytes - 256, k2_num_sms(),
+                                  (cudaStream_t)stream);
+        if (rc != -1)
+            return rc;
+    }
     if (one_per_cta) {
         // CTA b integrates item order[b] (or b) and retires: no queue
         A.counter = nullptr;
@@ -1208,6 +1392,11 @@ namespace dgb {
 int preload_integrate2d()
 {
     return preload(k_integrate2d<false>) + preload(k_integrate2d<true>) +
-           preload(k_integrate2d_pair) + preload(k_sched2d);
+           preload(k2w_kernel<1>(true)) +
+           preload(k2w_kernel<2>(true)) + preload(k2w_kernel<3>(true)) +
+           preload(k2w_kernel<4>(true)) + preload(k2w_kernel<5>(true)) +
+           preload(k2w_kernel<1>(false)) + preload(k2w_kernel<2>(false)) +
+           preload(k2w_kernel<3>(false)) + preload(k2w_kernel<4>(false)) +
+           preload(k2w_kernel<5>(false)) + preload(k_sched2d);
 }
 } // namespace dgb

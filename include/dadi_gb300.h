@@ -71,15 +71,12 @@ typedef struct {
     int use_old_timestep;        /* default 0 */
     int use_delj_trick;          /* default 0 */
     int gam_placement;           /* batched engine: 0 auto, 1 shared memory, 2 workspace */
-    int threads;                 /* batched engine: threads per CTA, 0 auto (the fewest
-                                    warps, 2-4, that give every line of the largest grid a
-                                    lane; for a launch over one grid of 73-128 points, two
-                                    work items per CTA on ceil(2L/32) warps where that fills
-                                    the lanes better), or 64 / 96 /
-                                    128 where that many threads hold every line (else
-                                    auto), one item per CTA, or -2: as auto but with two
-                                    items per CTA at any L where that fills the warps'
-                                    lanes better */
+    int threads;                 /* batched engine: 0 (or -2) auto -- a lane per line of the
+                                    largest grid for the solves and as many for the factors
+                                    of the next sweep -- or 64 / 96 / 128 threads per CTA,
+                                    one lane for both, where that many threads hold every
+                                    line (else the fewest warps, 2-4, that do); the delj
+                                    trick and gam_placement 1 always take the latter */
     int line_solver;             /* batched N-dimensional engine: 0 Thomas, one line per
                                     thread (dadi/tridiag.c:14-34); 1 parallel cyclic
                                     reduction, one warp per line (L <= 128); 2 partitioned

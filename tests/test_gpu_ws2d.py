@@ -1,0 +1,60 @@
+"""k_integrate2d_ws (each sweep's factors on other warps than its solves)
+against k_integrate2d, which runs them one after the other: the same bits, at
+the edges of its warps of lines, its load batches and its ring of step
+scalars, and in both forms of the solve."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _sets(n, steps, seed):
+    """IM sets of about `steps` steps with growth, migration and a set without
+    migration (exact zero couplings at the boundary rows)."""
+    rng = np.random.default_rng(seed)
+    p = np.stack([rng.uniform(0.3, 0.7, n), rng.uniform(0.3, 3, n), rng.uniform(0.3, 3, n),
+                  np.full(n, steps * 1e-4), rng.uniform(9, 10, n), rng.uniform(0, 9, n)], axis=1)
+    p[-1, 4:] = 0
+    return p
+
+
+def _both(L, rec):
+    from dadi_gb300 import batch
+    eng = batch.Batch2D((L,), (4, 4))
+    out = []
+    for threads in (0, 128):  # 128: one warp for both
+        eng.threads = threads
+        phis, status = eng.integrate(rec)
+        assert int(status.abs().sum()) == 0
+        out.append(phis[0].cpu().numpy())
+    return out
+
+
+@pytest.mark.parametrize("L", [3, 4, 5, 12, 13, 31, 32, 33, 63, 64, 65, 96, 97, 128, 129, 159,
+                               160, 161])
+def test_same_bits_at_every_warp_count(cuda_lib, L):
+    from dadi_gb300 import batch
+    got, want = _both(L, batch.im_instances(_sets(3, 40 if L < 100 else 18, L)))
+    assert np.array_equal(got, want)
+
+
+def test_same_bits_across_the_scalar_ring_and_masks(cuda_lib):
+    """Schedules of 0 to 130 steps in one queue, frozen axes and suppressed
+    mutations, selection."""
+    from dadi_gb300 import batch
+    p = _sets(24, 60, 1)
+    p[:, 3] *= np.linspace(0, 2.2, 24)
+    p[8:16, 4:] = 0
+    rec = batch.im_instances(p)
+    rec["frozen"][8:16] = np.arange(8) % 4
+    rec["nomut"][12:20] = np.arange(8) % 4
+    rec["gamma"][::3, 0, 1] = -30.0
+    got, want = _both(47, rec)
+    assert np.array_equal(got, want)
+
+
+def test_same_bits_where_the_solves_form_a_again(cuda_lib):
+    """More CTAs than have their coefficients in L2."""
+    from dadi_gb300 import batch
+    got, want = _both(130, batch.im_instances(_sets(170, 6, 2)))
+    assert np.array_equal(got, want)
