@@ -284,25 +284,6 @@ struct ADShared {
     int item;
 };
 
-__device__ __forceinline__ void ad_axis_scalars(AxisScalars &s, int a, const double *row,
-                                                const GridVecs &g, int L)
-{
-    double dt = row[0];
-    s.dt = dt;
-    s.nu = row[row_nu(2, a)];
-    s.inv_nu = 1.0 / s.nu;
-    s.gamma = row[row_gamma(2, a)];
-    s.h = row[row_h(2, a)];
-    double m = row[row_mig(2, a, 1 - a)];
-    s.msum = m;
-    s.mig[a] = 0;
-    s.mig[1 - a] = m;
-    s.B1s = 0.5 * (dt * g.dfac[0]);
-    s.B1e = -0.5 * (dt * g.dfac[L - 1]);
-    corner_bc(2, a, s.mig, s.nu, s.gamma, s.h, g.x[0], g.x[L - 1], g.dx[0], g.dx[L - 2], dt,
-              s.bcs, s.bce);
-}
-
 // Per-step setup shared by the recomputation and the backward step: axis
 // scalars, injection value and (with transposed) the derivative row.
 __device__ void ad_step_setup(ADShared &S, ADVecs &V, const GridVecs &g, int L, const double *row,
@@ -310,7 +291,7 @@ __device__ void ad_step_setup(ADShared &S, ADVecs &V, const GridVecs &g, int L, 
 {
     const int tid = threadIdx.x;
     if (tid < 2)
-        ad_axis_scalars(S.ax[tid], tid, row, g, L);
+        axis_scalars_2d(S.ax[tid], tid, row, g, L);
     else if (tid == 2) {
         S.inj = inject_value(2, row[0], row[1], g.x[0], g.x[1], g.x[2]);
         S.dinj_dt = inject_value(2, 1.0, row[1], g.x[0], g.x[1], g.x[2]);

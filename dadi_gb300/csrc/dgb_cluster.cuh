@@ -19,8 +19,10 @@
 //   C2_YSEG segments on C2_YSEG threads (16 rows fill 128 lanes) and solved
 //   the same way with CTA barriers.
 //
-// Both are called by every thread of the CTA (and, for x, of every CTA of
-// the cluster): they contain the barriers.  Default delta_j rows only.
+// Both are called by the first C2_THREADS threads of the CTA (and, for x, of
+// every CTA of the cluster): they contain the barriers.  Further threads of
+// the CTA pass the two cluster barriers of c2_sweep_x on their own.  Default
+// delta_j rows only.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -28,7 +30,8 @@
 
 namespace dgb {
 
-constexpr int C2_THREADS = 128;
+constexpr int C2_THREADS = 128; // that solve
+constexpr int C2_BAR = 1;       // their barrier
 constexpr int C2_ROWS = 16; // rows per CTA at most
 constexpr int C2_YSEG = 8;  // segments per row in the y sweep
 constexpr int C2_XROW = 6;  // exported values per column: A' C' D' al ga de
@@ -144,7 +147,7 @@ __device__ __forceinline__ void c2_sweep_x(cooperative_groups::cluster_group &cl
             blk[p * pitch + j] =
                 fma(-ga[p * L + j], xl, fma(-al[p * L + j], xf, blk[p * pitch + j]));
     }
-    __syncthreads();
+    bar_group(C2_BAR, C2_THREADS);
 }
 
 // The y sweep of the CTA's rows; al, ga: L x C2_ROWS scratch ([c][p]); yr:
@@ -210,7 +213,7 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
         r8[1 * C2_ROWS] = xc;
         r8[2 * C2_ROWS] = xd;
     }
-    __syncthreads();
+    bar_group(C2_BAR, C2_THREADS);
     if (live) {
         const double Ap = r8[0], Cp = r8[C2_ROWS], Dp = r8[2 * C2_ROWS];
         const double alq = r8[3 * C2_ROWS], gaq = r8[4 * C2_ROWS], deq = r8[5 * C2_ROWS];
@@ -226,7 +229,7 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
         r8[5 * C2_ROWS] = -gaq * Cn;
         r8[6 * C2_ROWS] = fma(-gaq, Dn, fma(-alq, Dp, deq));
     }
-    __syncthreads();
+    bar_group(C2_BAR, C2_THREADS);
     if (live && q == 0) {
         double gm[C2_YSEG], z[C2_YSEG];
         double gq = 0, u = 0;
@@ -247,7 +250,7 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
         for (int k = 0; k < C2_YSEG; k++)
             yr[((size_t)k * C2_YSLOT + 7) * C2_ROWS + p] = z[k];
     }
-    __syncthreads();
+    bar_group(C2_BAR, C2_THREADS);
     if (live) {
         const double xl = r8[7 * C2_ROWS];
         const double zp = q ? r8[7 * C2_ROWS - C2_YSLOT * C2_ROWS] : 0.0;
@@ -257,7 +260,7 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
         for (int c = s0 + 1; c < s0 + ml - 1; c++)
             ph[c] = fma(-ga[c * C2_ROWS + p], xl, fma(-al[c * C2_ROWS + p], xf, ph[c]));
     }
-    __syncthreads();
+    bar_group(C2_BAR, C2_THREADS);
 }
 
 } // namespace dgb

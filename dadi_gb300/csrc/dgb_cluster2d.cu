@@ -55,21 +55,30 @@ struct C2Args {
     int ckpt_every;
 };
 
+// The step scalars and per-axis vectors of step k + 1 are formed by C2_PREP
+// further threads of every CTA while the first C2_THREADS solve step k (some
+// 40 FP64 instructions in a row for the vectors, as many again in the scalars'
+// divisions).  Microseconds per step on 8 CTAs, formed between the steps /
+// beside them: L = 50 21.9 / 17.7, 60 23.1 / 19.0, 80 26.9 / 21.7, 100 30.6 /
+// 26.1, 120 33.2 / 29.1.
+constexpr int C2_PREP = 128;
+constexpr int C2_STEPS = 16; // steps whose scalars are formed at once
+
 struct C2Shared {
-    AxisScalars ax[2];
-    double inj;
+    AxisScalars ax[2 * C2_STEPS][2]; // ring over the steps
+    double inj[2 * C2_STEPS];
 };
 
 
 // Shared memory (doubles) of one CTA for grids of up to L points.
 __host__ __device__ inline size_t c2_smem_doubles(int L)
 {
-    return (size_t)C2_ROWS * c2_pitch(L) + 2 * (size_t)C2_ROWS * L + 16 * (size_t)L +
+    return (size_t)C2_ROWS * c2_pitch(L) + 2 * (size_t)C2_ROWS * L + 26 * (size_t)L +
            (size_t)C2_XROW * L + 2 * (size_t)L + (size_t)C2_YSLOT * C2_YSEG * C2_ROWS;
 }
 
 
-__global__ void __launch_bounds__(C2_THREADS) k_integrate2d_cluster(C2Args A)
+__global__ void __launch_bounds__(C2_THREADS + C2_PREP) k_integrate2d_cluster(C2Args A)
 {
     extern __shared__ __align__(16) double smem[];
     __shared__ C2Shared Sh;
@@ -110,25 +119,24 @@ __global__ void __launch_bounds__(C2_THREADS) k_integrate2d_cluster(C2Args A)
     g.xInt = q0 + 3 * L;
     g.ih = q0 + 4 * L;
     g.dx = q0 + 5 * L;
-    AxisVecs v[2];
-    v[0].A1 = q0 + 6 * L;
-    v[0].A0 = q0 + 7 * L;
-    v[0].C1 = q0 + 8 * L;
-    v[0].C0 = q0 + 9 * L;
-    v[0].B0 = q0 + 10 * L;
-    v[1].A1 = q0 + 11 * L;
-    v[1].A0 = q0 + 12 * L;
-    v[1].C1 = q0 + 13 * L;
-    v[1].C0 = q0 + 14 * L;
-    v[1].B0 = q0 + 15 * L;
-    for (int a = 0; a < 2; a++)
-        v[a].G = v[a].Pv = v[a].Qv = v[a].VI = v[a].DF = nullptr;
-    double *xr = q0 + 16 * L;             // exported rows of the x segments, [k][j]
+    // the vectors of axis a in steps of parity k
+    auto vecs = [&](int k, int a) {
+        double *w = q0 + (6 + 10 * (k & 1) + 5 * a) * (size_t)L;
+        AxisVecs v;
+        v.A1 = w;
+        v.A0 = w + L;
+        v.C1 = w + 2 * L;
+        v.C0 = w + 3 * L;
+        v.B0 = w + 4 * L;
+        v.G = v.Pv = v.Qv = v.VI = v.DF = nullptr;
+        return v;
+    };
+    double *xr = q0 + 26 * L;             // exported rows of the x segments, [k][j]
     double *zin = xr + C2_XROW * L;       // z of this segment and of the one above, [2][j]
     double *yr = zin + 2 * L;             // y sweep slots, [(q * C2_YSLOT + k) * C2_ROWS + p]
 
     // grid constants and this CTA's rows of the initial density
-    for (int i = tid; i < L; i += C2_THREADS) {
+    for (int i = tid; i < L; i += blockDim.x) {
         const double x = xx[i];
         g.x[i] = x;
         g.xv[i] = x * (1. - x);
@@ -139,12 +147,12 @@ __global__ void __launch_bounds__(C2_THREADS) k_integrate2d_cluster(C2Args A)
             g.xInt[i] = 0.5 * (xx[i + 1] + x);
         }
     }
-    for (int idx = tid; idx < m * L; idx += C2_THREADS) {
+    for (int idx = tid; idx < m * L; idx += blockDim.x) {
         const int p = idx / L, c = idx - p * L;
         blk[p * pitch + c] = phi_g[(size_t)(R0 + p) * L + c];
     }
     __syncthreads();
-    for (int i = tid; i < L; i += C2_THREADS)
+    for (int i = tid; i < L; i += blockDim.x)
         g.dfac[i] = (i == 0)       ? 2. / g.dx[0]
                     : (i == L - 1) ? 2. / g.dx[L - 2]
                                    : 2. / (g.dx[i] + g.dx[i - 1]);
@@ -152,57 +160,61 @@ __global__ void __launch_bounds__(C2_THREADS) k_integrate2d_cluster(C2Args A)
     const int j0 = (g.x[0] == 0.0) ? 0 : -1;
     const int j1 = (g.x[L - 1] == 1.0) ? L - 1 : -1;
 
-    for (int step = 0; step < nsteps; step++) {
-        const double *row = table + (size_t)step * 11;
-        if (ck && step % A.ckpt_every == 0) {
-            // this CTA's rows of phi before the step
-            double *c = ck + (size_t)(step / A.ckpt_every) * L * L + (size_t)R0 * L;
-            for (int idx = tid; idx < m * L; idx += C2_THREADS) {
-                const int p = idx / L, q = idx - p * L;
-                c[idx] = blk[p * pitch + q];
+    const bool solves = tid < C2_THREADS;
+    for (int step = -1; step < nsteps; step++) {
+        if (!solves) {
+            const int q = tid - C2_THREADS, n = step + 1;
+            if (step >= 0 && !(frozen & 1)) {
+                cluster.sync(); // c2_sweep_x's two
+                cluster.sync();
             }
-        }
-        if (tid < 2) {
-            AxisScalars &s = Sh.ax[tid];
-            const int a = tid;
-            const double dt = row[0];
-            s.dt = dt;
-            s.nu = row[row_nu(2, a)];
-            s.inv_nu = 1.0 / s.nu;
-            s.gamma = row[row_gamma(2, a)];
-            s.h = row[row_h(2, a)];
-            const double mg = row[row_mig(2, a, 1 - a)];
-            s.msum = mg;
-            s.mig[a] = 0;
-            s.mig[1 - a] = mg;
-            s.B1s = 0.5 * (dt * g.dfac[0]);
-            s.B1e = -0.5 * (dt * g.dfac[L - 1]);
-            corner_bc(2, a, s.mig, s.nu, s.gamma, s.h, g.x[0], g.x[L - 1], g.dx[0], g.dx[L - 2],
-                      dt, s.bcs, s.bce);
-        } else if (tid == 2) {
-            Sh.inj = inject_value(2, row[0], row[1], g.x[0], g.x[1], g.x[2]);
+            if (n < nsteps) {
+                if (n % C2_STEPS == 0) {
+                    const int st = n + (q >> 1);
+                    const double *row = table + (size_t)st * 11;
+                    if (q < 2 * C2_STEPS && st < nsteps) {
+                        axis_scalars_2d(Sh.ax[st % (2 * C2_STEPS)][q & 1], q & 1, row, g, L);
+                        if (!(q & 1))
+                            Sh.inj[st % (2 * C2_STEPS)] =
+                                inject_value(2, row[0], row[1], g.x[0], g.x[1], g.x[2]);
+                    }
+                    bar_group(C2_BAR + 1, C2_PREP);
+                }
+                for (int t = q; t < 2 * L; t += C2_PREP) {
+                    const int a = t >= L, i = t - a * L;
+                    AxisVecs v = vecs(n, a);
+                    build_axis_entry(i, L, g, Sh.ax[n % (2 * C2_STEPS)][a], 1.0, false, v);
+                }
+            }
+        } else if (step >= 0) {
+            if (ck && step % A.ckpt_every == 0) {
+                // this CTA's rows of phi before the step
+                double *c = ck + (size_t)(step / A.ckpt_every) * L * L + (size_t)R0 * L;
+                for (int idx = tid; idx < m * L; idx += C2_THREADS) {
+                    const int p = idx / L, q = idx - p * L;
+                    c[idx] = blk[p * pitch + q];
+                }
+                bar_group(C2_BAR, C2_THREADS);
+            }
+            const AxisScalars *ax = Sh.ax[step % (2 * C2_STEPS)];
+            if (tid == 0 && rank == 0) {
+                // rows 0 and 1 are this CTA's (m >= 3)
+                const double inj = Sh.inj[step % (2 * C2_STEPS)];
+                if (!(frozen & 1) && !(nomut & 1))
+                    blk[1 * pitch + 0] += inj;
+                if (!(frozen & 2) && !(nomut & 2))
+                    blk[0 * pitch + 1] += inj;
+            }
+            bar_group(C2_BAR, C2_THREADS);
+            if (!(frozen & 1))
+                c2_sweep_x(cluster, S, rank, blk, pitch, L, R0, m, al, ga, xr, zin,
+                           vecs(step, 0), ax[0], g, j0, j1);
+            if (!(frozen & 2))
+                c2_sweep_y(blk, pitch, L, R0, m, al, ga, yr, vecs(step, 1), ax[1], g, j0, j1);
         }
         __syncthreads();
-        for (int t = tid; t < 2 * L; t += C2_THREADS) {
-            const int a = t >= L, i = t - a * L;
-            build_axis_entry(i, L, g, Sh.ax[a], 1.0, false, v[a]);
-        }
-        if (tid == 0 && rank == 0) {
-            // rows 0 and 1 are this CTA's (m >= 3)
-            if (!(frozen & 1) && !(nomut & 1))
-                blk[1 * pitch + 0] += Sh.inj;
-            if (!(frozen & 2) && !(nomut & 2))
-                blk[0 * pitch + 1] += Sh.inj;
-        }
-        __syncthreads();
-
-        if (!(frozen & 1))
-            c2_sweep_x(cluster, S, rank, blk, pitch, L, R0, m, al, ga, xr, zin, v[0], Sh.ax[0],
-                       g, j0, j1);
-        if (!(frozen & 2))
-            c2_sweep_y(blk, pitch, L, R0, m, al, ga, yr, v[1], Sh.ax[1], g, j0, j1);
     }
-    for (int idx = tid; idx < m * L; idx += C2_THREADS) {
+    for (int idx = tid; idx < m * L; idx += blockDim.x) {
         const int p = idx / L, c = idx - p * L;
         phi_g[(size_t)(R0 + p) * L + c] = blk[p * pitch + c];
     }
@@ -236,7 +248,7 @@ static int c2_launch(const C2Args &A, int nclusters, int cluster, int Lmax, cuda
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(cluster * nclusters), 1, 1);
-    cfg.blockDim = dim3(C2_THREADS, 1, 1);
+    cfg.blockDim = dim3(C2_THREADS + C2_PREP, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];

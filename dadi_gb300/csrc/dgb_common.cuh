@@ -349,6 +349,33 @@ DGB_HD void corner_bc(int P, int axis, const double *mig, double nu, double gamm
     bce = (ml >= 0) ? dt * (-(-0.5 / nu - ml) * 2. / dxl) : 0.0;
 }
 
+// Scalars of axis a for one step from a parameter row (called by one lane
+// per axis so both axes cost one warp-wide instruction stream).
+__device__ __forceinline__ void axis_scalars_2d(AxisScalars &s, int a, const double *row,
+                                                const GridVecs &g, int L)
+{
+    double dt = row[0];
+    s.dt = dt;
+    s.nu = row[row_nu(2, a)];
+    s.inv_nu = 1.0 / s.nu;
+    s.gamma = row[row_gamma(2, a)];
+    s.h = row[row_h(2, a)];
+    double m = row[row_mig(2, a, 1 - a)];
+    s.msum = m;
+    s.mig[a] = 0;
+    s.mig[1 - a] = m;
+    s.B1s = 0.5 * (dt * g.dfac[0]);
+    s.B1e = -0.5 * (dt * g.dfac[L - 1]);
+    corner_bc(2, a, s.mig, s.nu, s.gamma, s.h, g.x[0], g.x[L - 1], g.dx[0], g.dx[L - 2], dt,
+              s.bcs, s.bce);
+}
+
+// Barrier of n threads of a CTA.
+__device__ __forceinline__ void bar_group(int id, int n)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
 // ------------------------------------------- the delj path's exact operations
 
 __device__ __forceinline__ double xm(double a, double b) { return __dmul_rn(a, b); }

@@ -126,27 +126,6 @@ __device__ __forceinline__ void k2_carve(double *smem, int Lmax, int pitch, bool
     }
 }
 
-// Scalars of axis a for one step from a parameter row (called by one lane
-// per axis so both axes cost one warp-wide instruction stream).
-__device__ __forceinline__ void k2_axis_scalars(AxisScalars &s, int a, const double *row,
-                                                const GridVecs &g, int L)
-{
-    double dt = row[0];
-    s.dt = dt;
-    s.nu = row[row_nu(2, a)];
-    s.inv_nu = 1.0 / s.nu;
-    s.gamma = row[row_gamma(2, a)];
-    s.h = row[row_h(2, a)];
-    double m = row[row_mig(2, a, 1 - a)];
-    s.msum = m;
-    s.mig[a] = 0;
-    s.mig[1 - a] = m;
-    s.B1s = 0.5 * (dt * g.dfac[0]);
-    s.B1e = -0.5 * (dt * g.dfac[L - 1]);
-    corner_bc(2, a, s.mig, s.nu, s.gamma, s.h, g.x[0], g.x[L - 1], g.dx[0], g.dx[L - 2], dt,
-              s.bcs, s.bce);
-}
-
 // Work item wid of a launch.
 struct K2Item {
     int wid, L, frozen, nomut, nsteps;
@@ -259,7 +238,7 @@ __global__ void __launch_bounds__(K2_THREADS) k_integrate2d(K2Args A)
             // ---- step scalars: lane a of warp 0 handles axis a, lane 2 the injection
             if (warp == 0) {
                 if (lane < 2)
-                    k2_axis_scalars(S.ax[lane], lane, row, g, L);
+                    axis_scalars_2d(S.ax[lane], lane, row, g, L);
                 else if (lane == 2)
                     S.inj = inject_value(2, row[0], row[1], g.x[0], g.x[1], g.x[2]);
             }
@@ -359,11 +338,6 @@ __host__ __device__ inline size_t k2w_slice_doubles(int L, bool keep_a)
 __host__ __device__ inline size_t k2w_smem_doubles(int L)
 {
     return (size_t)L * odd_pitch(L) + 6 * (size_t)L + 10 * (size_t)L;
-}
-
-__device__ __forceinline__ void bar_group(int id, int n)
-{
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
 // 1/bet and c * (1/bet).
@@ -577,7 +551,7 @@ __global__ void __launch_bounds__(32 * W * k2w_groups(W), W == 1 ? 5 : W == 2 ? 
                 const int st = n + (q >> 1);
                 const double *row = I.rows + (size_t)st * K2_ROW;
                 if (q < 2 * K2W_STEPS && st < I.nsteps)
-                    k2_axis_scalars(S.ax[st % (2 * K2W_STEPS)][q & 1], q & 1, row, g, L);
+                    axis_scalars_2d(S.ax[st % (2 * K2W_STEPS)][q & 1], q & 1, row, g, L);
                 if (q < 2 * K2W_STEPS && st < I.nsteps && !(q & 1))
                     S.inj[st % (2 * K2W_STEPS)] =
                         inject_value(2, row[0], row[1], g.x[0], g.x[1], g.x[2]);
