@@ -165,6 +165,73 @@ __device__ __forceinline__ double rcp_full(double x)
     return r;
 }
 
+// 1/x for x = m 2^E to 67 bits: r[2]:r[1]:r[0] = 2^96 / m (rcp_mant's, with
+// one more term of the series, before its rounding).
+__device__ __forceinline__ void rcp_wide(double x, unsigned (&r)[3])
+{
+    const unsigned xh = (unsigned)__double2hiint(x), xl = (unsigned)__double2loint(x);
+    const unsigned hx = (xh & 0xfffffu) | 0x100000u;
+    const double seed = rcp_seed(__hiloint2double((int)(hx + 0x3fe00000u), (int)xl));
+    const unsigned rho = (unsigned)__double2hiint(seed) - 0x3fd00000u;
+    const unsigned nr = 0u - rho;
+    const unsigned long long t = (unsigned long long)xl * nr;
+    const unsigned eh = (unsigned)(t >> 32) + hx * nr - xl;
+    const unsigned long long e = (unsigned long long)eh << 32 | (unsigned)t;
+    const int s = (int)__funnelshift_r((unsigned)t, eh, 23);
+    const int q = __mulhi(s, s);
+    const unsigned long long f = (unsigned long long)(unsigned)q * 32u + e +
+                                 (unsigned long long)(long long)(__mulhi(s, q) >> 13);
+    const unsigned r4 = rho << 2;
+    const unsigned long long w = (unsigned long long)r4 * (unsigned)f;
+    const unsigned long long y =
+        (unsigned long long)((long long)(int)r4 * (int)(f >> 32)) +
+        ((unsigned long long)(rho << 11) << 32 | (unsigned)(w >> 32));
+    r[0] = (unsigned)w;
+    r[1] = (unsigned)y;
+    r[2] = (unsigned)(y >> 32);
+}
+
+// (The delj rows have five divisions a point: 64 IM sets at pts 40/50/60 took
+// 1.33 s with them on the FP64 pipe, 0.89 with div_full.)
+static __device__ __noinline__ double div_fp64(double x, double y) { return __ddiv_rn(x, y); }
+
+// x / y rounded as IEEE division rounds, from y's rcp_wide.  A quotient is
+// never half way between two doubles, and one within the error of it (one in
+// 2^11), or out of range, is left to the FP64 pipe (some 10 instructions).
+__device__ __forceinline__ double div_wide(double x, double y, const unsigned (&r)[3])
+{
+    const unsigned xh = (unsigned)__double2hiint(x), xl = (unsigned)__double2loint(x);
+    const unsigned yh = (unsigned)__double2hiint(y);
+    const unsigned mh = (xh & 0xfffffu) | 0x100000u;
+    const unsigned long long t1 = (unsigned long long)mh * r[1] + __umulhi(xl, r[1]);
+    const unsigned long long t2 = (unsigned long long)xl * r[2] +
+                                  ((unsigned long long)(unsigned)t1 + __umulhi(mh, r[0]));
+    const unsigned long long p = (unsigned long long)mh * r[2] +
+                                 ((unsigned long long)(unsigned)(t1 >> 32) + (unsigned)(t2 >> 32));
+    const unsigned w1 = (unsigned)t2, w2 = (unsigned)p, w3 = (unsigned)(p >> 32);
+    const unsigned sh = (w3 >> 20) ^ 1u;
+    const unsigned m1 = w1 << sh;
+    const unsigned long long m = ((unsigned long long)__funnelshift_l(w2, w3, sh) << 32 |
+                                  __funnelshift_l(w1, w2, sh)) +
+                                 (m1 >> 31);
+    const bool bad = (m1 - 0x7ff00000u < 0x200000u) | ((int)r[2] >= 0) |
+                     ((yh & 0x7fffffffu) - 0x37f00000u >= 0x10000000u) |
+                     ((xh & 0x7fffffffu) - 0x0c800000u >= 0x66000000u);
+    double q = __hiloint2double((int)((unsigned)(m >> 32) + (xh & 0xfff00000u) + 0x3fd00000u -
+                                      (yh & 0xfff00000u) + (w3 & 0x100000u)),
+                                (int)(unsigned)m);
+    if (bad)
+        q = div_fp64(x, y);
+    return q;
+}
+
+__device__ __forceinline__ double div_full(double x, double y)
+{
+    unsigned r[3];
+    rcp_wide(y, r);
+    return div_wide(x, y, r);
+}
+
 // x * y rounded as IEEE multiplication rounds (y an unpacked double).
 __device__ __forceinline__ double mul_full(double x, double y)
 {
@@ -381,7 +448,10 @@ __device__ __forceinline__ void bar_group(int id, int n)
 __device__ __forceinline__ double xm(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double xa(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double xs(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double xd(double a, double b) { return __ddiv_rn(a, b); }
+__device__ __forceinline__ double xd(double a, double b) { return div_full(a, b); }
+// xm on the integer pipes (b of ordinary size), for products that no chain
+// waits for.
+__device__ __forceinline__ double xmi(double a, double b) { return mul_full(a, b); }
 
 // Selection part of Mfunc (dadi/integration_shared.c:12-14) in the
 // reference's order: gamma * 2*(h + (1.-2*h)*x) * x*(1.-x).
@@ -519,10 +589,15 @@ __device__ __forceinline__ void solve_line(TP *__restrict__ ph, int sp, TG *__re
 // in the reference's order.
 __device__ __forceinline__ double delj_of(double MInt, double VInt, double dx)
 {
-    const double wj = xm(xm(2.0, MInt), dx);
+    const double wj = xmi(MInt, 2.0 * dx); // (2 MInt) dx: doubling is exact
     const double epsj = exp(xd(wj, VInt));
-    if ((epsj != 1.0) && (wj != 0))
-        return xd(xs(xa(xm(-epsj, wj), xm(epsj, VInt)), VInt), xs(wj, xm(epsj, wj)));
+    // epsj != 1.0 && wj != 0 (not on the FP64 pipe, which a comparison takes
+    // longer than a fused multiply-add)
+    if (__double_as_longlong(epsj) != 0x3ff0000000000000ll && __double_as_longlong(wj) << 1 != 0)
+    {
+        const double ew = xmi(wj, epsj);
+        return xd(xs(xa(-ew, xmi(VInt, epsj)), VInt), xs(wj, ew));
+    }
     return 0.5;
 }
 

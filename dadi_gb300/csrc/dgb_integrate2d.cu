@@ -622,6 +622,262 @@ __global__ void __launch_bounds__(32 * W * k2w_groups(W), W == 1 ? 5 : W == 2 ? 
     }
 }
 
+// ------------------------------- the delj trick's coefficients ahead of the sweep
+
+// k_integrate2d<true> with delta_j and the intervals' coefficients (at, ct of
+// solve_line_delj: an exponential, two divisions and some 15 further FP64
+// instructions per interval and line, none of which depends on the row before
+// or on the density) formed one sweep ahead by k2d_groups(W) W further warps,
+// interval i by group i mod k2d_groups(W), and handed over through the
+// workspace.  What is left to the solve warps is the recurrence.  With the
+// divisions and the products that no chain waits for on the integer pipes
+// (div_wide, mul_full) some 40 FP64 instructions remain per point; from three
+// warps of lines on they fill the FP64 pipe, whatever the groups.  Every
+// operation is solve_line_delj's, so the results are bitwise the same.
+// Measured, microseconds per step of one grid with one warp for both / with
+// this kernel: L = 31 135 / 46, 60 256 / 103, 90 384 / 206, 128 544 / 359.
+constexpr __host__ __device__ int k2d_groups(int W)
+{
+    return W == 1 ? 8 : W == 2 ? 6 : W == 3 ? 5 : W == 4 ? 4 : 3;
+}
+
+__host__ __device__ inline size_t k2d_smem_doubles(int L)
+{
+    return (size_t)L * odd_pitch(L) + 6 * (size_t)L + 8 * (size_t)L;
+}
+
+// Workspace of one CTA: [axis][the four arrays of k2d_solve][row][line], then
+// the couplings of the sweep being solved.
+__host__ __device__ inline size_t k2d_slice_doubles(int L) { return (size_t)9 * L * k2w_pitch(L); }
+
+// solve_line_delj from the products of its intervals' at and ct with dfactor,
+// arrays f + k * stride, row i at i * LP: k = 0 a_i = -DF_i at_{i-1}, 1 1/dt +
+// DF_i ct_{i-1}, 2 DF_i at_i, 3 c_i = -DF_i ct_i; row 0 has the last two.
+__device__ __forceinline__ void k2d_solve(double *__restrict__ ph, int sp,
+                                          double *__restrict__ gm,
+                                          const double *__restrict__ f, size_t stride, int LP,
+                                          int L, double mo, double o, bool c0, bool c1,
+                                          const GridVecs &gv, const AxisScalars &s)
+{
+    constexpr int B = 3;
+    auto mfun = [&](double x, double sel) { return xa(xm(mo, xs(o, x)), sel); };
+    const double dt = s.dt;
+    unsigned rdt[3], rb[3];
+    rcp_wide(dt, rdt);
+    double fn[4][B]; // the next rows'
+    auto load = [&](int i) {
+#pragma unroll
+        for (int k = 0; k < B; k++)
+#pragma unroll
+            for (int n = 0; n < 4; n++)
+                fn[n][k] = __ldcg(f + n * stride + min(i + k, n < 2 ? L - 1 : L - 2) * LP);
+    };
+    double cprev = __ldcg(f + 3 * stride);
+    double bet = xa(xd(1.0, dt), __ldcg(f + 2 * stride));
+    load(1);
+    if (c0) {
+        const double mf = mfun(gv.x[0], msel_ref(gv.x[0], s.gamma, s.h));
+        if (mf <= 0)
+            bet = xa(bet, xd(xm(xs(xd(0.5, s.nu), mf), 2.0), gv.dx[0]));
+    }
+    rcp_wide(bet, rb);
+    double u = div_wide(div_wide(ph[0], dt, rdt), bet, rb);
+    ph[0] = u;
+    for (int i0 = 1; i0 < L; i0 += B) {
+        double fv[4][B], pv[B];
+#pragma unroll
+        for (int k = 0; k < B; k++) {
+#pragma unroll
+            for (int n = 0; n < 4; n++)
+                fv[n][k] = fn[n][k];
+            pv[k] = ph[min(i0 + k, L - 1) * sp];
+        }
+        load(i0 + B);
+#pragma unroll
+        for (int k = 0; k < B; k++) {
+            const int i = i0 + k;
+            if (i >= L)
+                break;
+            const double a = fv[0][k];
+            double bb = fv[1][k];
+            if (i < L - 1) {
+                bb = xa(bb, fv[2][k]);
+            } else if (c1) {
+                const double ml = mfun(gv.x[L - 1], msel_ref(gv.x[L - 1], s.gamma, s.h));
+                if (ml >= 0)
+                    bb = xa(bb, xd(xm(-xs(-xd(0.5, s.nu), ml), 2.0), gv.dx[L - 2]));
+            }
+            const double g = div_wide(cprev, bet, rb);
+            gm[i * LP] = g;
+            bet = xs(bb, xm(a, g));
+            rcp_wide(bet, rb);
+            u = div_wide(xs(div_wide(pv[k], dt, rdt), xm(a, u)), bet, rb);
+            ph[i * sp] = u;
+            cprev = fv[3][k];
+        }
+    }
+    constexpr int C = 8;
+    int i = L - 2;
+    for (; i >= C - 1; i -= C) {
+        double g[C], p[C];
+#pragma unroll
+        for (int k = 0; k < C; k++) {
+            g[k] = __ldcg(gm + (i - k + 1) * LP);
+            p[k] = ph[(i - k) * sp];
+        }
+#pragma unroll
+        for (int k = 0; k < C; k++) {
+            u = xs(p[k], xm(g[k], u));
+            ph[(i - k) * sp] = u;
+        }
+    }
+    for (; i >= 0; i--) {
+        u = xs(ph[i * sp], xm(__ldcg(gm + (i + 1) * LP), u));
+        ph[i * sp] = u;
+    }
+}
+
+template <int W>
+__global__ void __launch_bounds__(32 * W * (1 + k2d_groups(W)), 1) k_integrate2d_delj(K2Args A)
+{
+    extern __shared__ __align__(16) double smem[];
+    __shared__ K2WShared S;
+    constexpr int ng = 32 * W, NG = k2d_groups(W), nc = NG * ng;
+    const int tid = threadIdx.x;
+    const int group = tid / ng, q = tid - group * ng; // group 0 solves
+    const int pitch = odd_pitch(A.Lmax);
+    double *phi = smem;
+    GridVecs g;
+    double *p = smem + (size_t)A.Lmax * pitch;
+    g.x = p; p += A.Lmax;
+    g.xv = p; p += A.Lmax;
+    g.dfac = p; p += A.Lmax;
+    g.xInt = p; p += A.Lmax;
+    g.ih = p; p += A.Lmax;
+    g.dx = p; p += A.Lmax;
+    double *vec = p; // G, Pv, Qv, VI of the sweep being prepared
+    double *slice = A.gam_glob + (size_t)blockIdx.x * k2d_slice_doubles(A.Lmax);
+
+    for (int iter = 0;; iter++) {
+        if (tid == 0)
+            S.item = A.counter ? atomicAdd(A.counter, 1) : (iter == 0 ? (int)blockIdx.x : A.nwork);
+        __syncthreads();
+        const int w = S.item;
+        if (w >= A.nwork)
+            break;
+        const K2Item I = k2_item(A, A.order ? A.order[w] : w);
+        const int L = I.L, LP = k2w_pitch(L);
+        const size_t stride = (size_t)L * LP;
+        for (int i = tid; i < L; i += blockDim.x) {
+            double x = I.xx[i];
+            g.x[i] = x;
+            g.xv[i] = x * (1. - x);
+            if (i < L - 1) {
+                double d = I.xx[i + 1] - x;
+                g.dx[i] = d;
+                g.ih[i] = 1.0 / (2 * d);
+                g.xInt[i] = 0.5 * (I.xx[i + 1] + x);
+            }
+        }
+        for (int idx = tid; idx < L * L; idx += blockDim.x) {
+            int r = idx / L, c = idx - r * L;
+            phi[r * pitch + c] = I.src[idx];
+        }
+        __syncthreads();
+        for (int i = tid; i < L; i += blockDim.x) {
+            if (i == 0)
+                g.dfac[i] = 2. / g.dx[0];
+            else if (i == L - 1)
+                g.dfac[i] = 2. / g.dx[L - 2];
+            else
+                g.dfac[i] = 2. / (g.dx[i] + g.dx[i - 1]);
+        }
+        __syncthreads();
+        const int j0 = (g.x[0] == 0.0) ? 0 : -1;
+        const int j1 = (g.x[L - 1] == 1.0) ? L - 1 : -1;
+        const int nsw = 2 * I.nsteps; // sweep m: axis m & 1 of step m >> 1
+        for (int m = -1; m < nsw; m++) {
+            if (group) {
+                // the coefficients of sweep m + 1
+                const int r = tid - ng, a = (m + 1) & 1, n = (m + 1) >> 1;
+                if (m + 1 < nsw) {
+                    if (a == 0 && n % K2W_STEPS == 0) {
+                        const int st = n + (r >> 1);
+                        const double *row = I.rows + (size_t)st * K2_ROW;
+                        if (r < 2 * K2W_STEPS && st < I.nsteps) {
+                            axis_scalars_2d(S.ax[st % (2 * K2W_STEPS)][r & 1], r & 1, row, g, L);
+                            if (!(r & 1))
+                                S.inj[st % (2 * K2W_STEPS)] =
+                                    inject_value(2, row[0], row[1], g.x[0], g.x[1], g.x[2]);
+                        }
+                        bar_group(2, nc);
+                    }
+                    if (!(I.frozen >> a & 1)) {
+                        const AxisScalars &s = S.ax[n % (2 * K2W_STEPS)][a];
+                        for (int t = r; t < 4 * (L - 1); t += nc) {
+                            const int k = t / (L - 1), i = t - k * (L - 1);
+                            const double d2 = xm(2.0, g.dx[i]);
+                            vec[k * L + i] =
+                                k == 0   ? msel_ref(g.xInt[i], s.gamma, s.h)
+                                : k == 1 ? xd(vfunc_ref(g.x[i], s.nu, 0.0), d2)
+                                : k == 2 ? xd(vfunc_ref(g.x[i + 1], s.nu, 0.0), d2)
+                                         : vfunc_ref(g.xInt[i], s.nu, 0.0);
+                        }
+                        bar_group(2, nc);
+                        double *f = slice + (size_t)a * 4 * stride + q;
+                        if (q < L) {
+                            const double mo = s.mig[1 - a], o = g.x[q], idt = xd(1.0, s.dt);
+                            for (int i = group - 1; i < L - 1; i += NG) {
+                                const double Mk = xa(xmi(xs(o, g.xInt[i]), mo), vec[i]);
+                                const double d = delj_of(Mk, vec[3 * L + i], g.dx[i]);
+                                const double at = xa(xmi(Mk, d), vec[L + i]);
+                                const double ct = xa(xmi(-Mk, xs(1.0, d)), vec[2 * L + i]);
+                                const double d0 = g.dfac[i], d1 = g.dfac[i + 1];
+                                f[(i + 1) * LP] = -xmi(at, d1);
+                                f[stride + (i + 1) * LP] = xa(idt, xmi(ct, d1));
+                                f[2 * stride + i * LP] = xmi(at, d0);
+                                f[3 * stride + i * LP] = -xmi(ct, d0);
+                            }
+                        }
+                    }
+                }
+            } else if (m >= 0) {
+                const int a = m & 1, k = m >> 1;
+                const AxisScalars &s = S.ax[k % (2 * K2W_STEPS)][a];
+                if (a == 0) {
+                    if (A.ckpt && k % A.ckpt_every == 0) {
+                        double *c = A.ckpt + A.ckpt_off[I.wid] + (size_t)(k / A.ckpt_every) * L * L;
+                        for (int idx = q; idx < L * L; idx += ng) {
+                            int r = idx / L, cl = idx - r * L;
+                            c[idx] = phi[r * pitch + cl];
+                        }
+                        bar_group(1, ng);
+                    }
+                    if (q == 0) {
+                        const double inj = S.inj[k % (2 * K2W_STEPS)];
+                        if (!(I.frozen & 1) && !(I.nomut & 1))
+                            phi[1 * pitch + 0] += inj;
+                        if (!(I.frozen & 2) && !(I.nomut & 2))
+                            phi[0 * pitch + 1] += inj;
+                    }
+                    bar_group(1, ng);
+                }
+                if (!(I.frozen >> a & 1) && q < L) {
+                    k2d_solve(phi + (size_t)q * ((a == 0) ? 1 : pitch), (a == 0) ? pitch : 1,
+                              slice + 8 * stride + q, slice + (size_t)a * 4 * stride + q, stride,
+                              LP, L, s.mig[1 - a], g.x[q], q == j0, q == j1, g, s);
+                }
+            }
+            __syncthreads();
+        }
+        for (int idx = tid; idx < L * L; idx += blockDim.x) {
+            int r = idx / L, c = idx - r * L;
+            I.out[idx] = phi[r * pitch + c];
+        }
+        __syncthreads();
+    }
+}
+
 // ------------------------------------------------------- schedule pass
 
 // Walk the reference time loop of two_pops (dadi/Integration.py:346-386) for
@@ -904,8 +1160,8 @@ static int k2w_per_sm(long nwork, int sms)
 
 // Launch k_integrate2d_ws over A's work (queue counter already cleared, or
 // null: one item per CTA) on `sms` SMs with slices from `slices` on; -1 where
-// it does not apply: the delj trick, grids beyond five warps of lines or
-// shared memory, or too little workspace.  The solves take a from the
+// it does not apply: grids beyond five warps of lines or shared memory, or too
+// little workspace.  The solves take a from the
 // workspace where the slices of all CTAs stay within the L2 cache, and form it
 // again (one more FP64 instruction a point, a third less traffic) where not:
 // 152 grids of 128 points 90 us a step with a, 62 without; of 100 points 46
@@ -913,10 +1169,11 @@ static int k2w_per_sm(long nwork, int sms)
 static int k2w_launch(K2Args &A, void *slices, size_t bytes, int sms, cudaStream_t st)
 {
     const int warps = (A.Lmax + 31) / 32;
-    if (A.use_delj || warps > K2W_MAXWARPS)
+    if (warps > K2W_MAXWARPS)
         return -1;
-    const int threads = 32 * warps * k2w_groups(warps);
-    const size_t smem = k2w_smem_doubles(A.Lmax) * sizeof(double);
+    const int threads = 32 * warps * (A.use_delj ? 1 + k2d_groups(warps) : k2w_groups(warps));
+    const size_t smem = (A.use_delj ? k2d_smem_doubles(A.Lmax) : k2w_smem_doubles(A.Lmax)) *
+                        sizeof(double);
     int dev = 0, optin = 0, occ = 0, l2 = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
@@ -927,11 +1184,16 @@ static int k2w_launch(K2Args &A, void *slices, size_t bytes, int sms, cudaStream
         return -1;
     void (*(*const kernels[])(bool))(K2Args) = {k2w_kernel<1>, k2w_kernel<2>, k2w_kernel<3>,
                                                 k2w_kernel<4>, k2w_kernel<5>};
+    void (*const delj[])(K2Args) = {k_integrate2d_delj<1>, k_integrate2d_delj<2>,
+                                    k_integrate2d_delj<3>, k_integrate2d_delj<4>,
+                                    k_integrate2d_delj<5>};
     void (*kernel)(K2Args) = nullptr;
     long nblocks = 0;
-    for (int keep = 1; keep >= (k2w_groups(warps) == 3 ? 1 : 0); keep--) {
-        const size_t slice = k2w_slice_doubles(A.Lmax, keep) * sizeof(double);
-        kernel = kernels[warps - 1](keep);
+    for (int keep = 1; keep >= (A.use_delj || k2w_groups(warps) == 3 ? 1 : 0); keep--) {
+        const size_t slice =
+            (A.use_delj ? k2d_slice_doubles(A.Lmax) : k2w_slice_doubles(A.Lmax, keep)) *
+            sizeof(double);
+        kernel = A.use_delj ? delj[warps - 1] : kernels[warps - 1](keep);
         if (raise_smem_limit(kernel))
             return -1;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) !=
@@ -987,16 +1249,18 @@ int k2_integrate_table(double *phi, int L, const double *xx, const double *table
     return k2_launch(A, 1, bytes, st);
 }
 
-size_t k2_table_ws_bytes(int L) { return k2w_slice_doubles(L, true) * sizeof(double); }
+size_t k2_table_ws_bytes(int L) { return k2d_slice_doubles(L) * sizeof(double); }
 
 size_t k2_batch_ws_bytes(int Lmax, long nwork)
 {
     const int sms = k2_num_sms();
     const size_t scratch = (size_t)sms * 4 * Lmax * Lmax; // k_integrate2d, up to four CTAs per SM
     const int per_sm = std::min(k2w_per_sm(nwork, sms), Lmax <= 64 ? 5 : 2);
-    const size_t slices = k2w_slice_doubles(Lmax, true) *
-                          (size_t)std::min<long>((long)sms * per_sm, std::max<long>(nwork, 1));
-    return 256 + std::max(scratch, slices) * sizeof(double);
+    auto slices = [&](int ctas, size_t slice) {
+        return slice * (size_t)std::min<long>((long)sms * ctas, std::max<long>(nwork, 1));
+    };
+    return 256 + sizeof(double) * std::max({scratch, slices(per_sm, k2w_slice_doubles(Lmax, true)),
+                                            slices(1, k2d_slice_doubles(Lmax))});
 }
 
 // norder: integrate only the work items order[0 .. norder) (<= 0: all);
@@ -1371,6 +1635,8 @@ int preload_integrate2d()
            preload(k2w_kernel<4>(true)) + preload(k2w_kernel<5>(true)) +
            preload(k2w_kernel<1>(false)) + preload(k2w_kernel<2>(false)) +
            preload(k2w_kernel<3>(false)) + preload(k2w_kernel<4>(false)) +
-           preload(k2w_kernel<5>(false)) + preload(k_sched2d);
+           preload(k2w_kernel<5>(false)) + preload(k_integrate2d_delj<1>) +
+           preload(k_integrate2d_delj<2>) + preload(k_integrate2d_delj<3>) +
+           preload(k_integrate2d_delj<4>) + preload(k_integrate2d_delj<5>) + preload(k_sched2d);
 }
 } // namespace dgb

@@ -31,7 +31,8 @@ __global__ void k_rcp(const double *x, double *out, int n)
     if (i < n)
         out[i] = rcp_full(x[i]);
 }
-// u = t * (1/x), g = c * (1/x) by pivot and, after them, on doubles.
+// u = t * (1/x), g = c * (1/x) by pivot, t / x by div_full and c * x by
+// mul_full and, after them, on doubles.
 __global__ void k_pivot(const double *xtc, double *out, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -41,10 +42,10 @@ __global__ void k_pivot(const double *xtc, double *out, int n)
     double u, g;
     pivot(x, t, c, u, g);
     const double2 d = pivot_fp64(x, t, c);
-    out[i] = u;
-    out[(size_t)n + i] = g;
-    out[2 * (size_t)n + i] = d.x;
-    out[3 * (size_t)n + i] = d.y;
+    const double v[8] = {u, g, div_full(t, x), mul_full(c, x),
+                         d.x, d.y, __ddiv_rn(t, x), __dmul_rn(c, x)};
+    for (int k = 0; k < 8; k++)
+        out[k * (size_t)n + i] = v[k];
 }
 } // namespace dgb
 

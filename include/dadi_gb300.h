@@ -609,8 +609,9 @@ int dgb_integrate2d_noalloc(double *phi, int L, const double *xx, const double *
  * dgb_probe_rcp: out[i] = the kernels' refined reciprocal of x[i] (device),
  * so tests can check it against correctly rounded division.
  * dgb_probe_pivot: for xtc = x[n], t[n], c[n] (device), out = t * (1/x),
- * c * (1/x) as the sweeps' integer arithmetic gives them, then the same two
- * as FP64 instructions give them (4 n doubles), so tests can compare the bits. */
+ * c * (1/x), t / x and c * x as the sweeps' integer arithmetic gives them,
+ * then the same four as FP64 instructions give them (8 n doubles), so tests
+ * can compare the bits. */
 int dgb_probe_fp64_fma(double *out, int blocks, int threads, int iters, int active_lanes,
                        void *stream);
 int dgb_probe_rcp(const double *x, double *out, int n, void *stream);

@@ -44,8 +44,8 @@ def _pivot_inputs(kind, n):
 
 @pytest.mark.parametrize("kind", ["pivots", "wide", "short mantissas", "any bits"])
 def test_integer_pivot_gives_the_bits_of_the_doubles(cuda_lib, kind):
-    """t * (1/x) and c * (1/x) on the integer pipes are, bit for bit, what the
-    FP64 instructions give (rounding, signs, and every value that leaves the
+    """t * (1/x), c * (1/x), t / x and c * x on the integer pipes are, bit for
+    bit, what the FP64 instructions give (rounding, signs, and every value that leaves the
     integers' range: zeros, subnormals, overflows, infinities; NaN as NaN)."""
     import torch
     from dadi_gb300 import _lib
@@ -53,11 +53,11 @@ def test_integer_pivot_gives_the_bits_of_the_doubles(cuda_lib, kind):
     with np.errstate(all="ignore"):
         xtc = np.concatenate(_pivot_inputs(kind, n))
     d = torch.from_numpy(xtc).cuda()
-    o = torch.empty(4 * n, dtype=torch.float64, device="cuda")
+    o = torch.empty(8 * n, dtype=torch.float64, device="cuda")
     _lib.check(cuda_lib.dgb_probe_pivot(_lib.dptr(d), _lib.dptr(o), n,
                                         _lib.stream_handle(torch)), "pivot")
     o = o.cpu().numpy()
-    got, want = o[:2 * n], o[2 * n:]
+    got, want = o[:4 * n], o[4 * n:]
     same = (got.view(np.int64) == want.view(np.int64)) | (np.isnan(got) & np.isnan(want))
     assert same.all()
 

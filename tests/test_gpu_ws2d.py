@@ -1,7 +1,8 @@
-"""k_integrate2d_ws (each sweep's factors on other warps than its solves)
-against k_integrate2d, which runs them one after the other: the same bits, at
-the edges of its warps of lines, its load batches and its ring of step
-scalars, and in both forms of the solve."""
+"""k_integrate2d_ws and, under the delj trick, k_integrate2d_delj (each sweep's
+factors or coefficients on other warps than its solves) against
+k_integrate2d, which runs them one after the other: the same bits, at the
+edges of their warps of lines, load batches and ring of step scalars, and in
+both forms of the solve."""
 import numpy as np
 import pytest
 
@@ -38,10 +39,26 @@ def test_same_bits_at_every_warp_count(cuda_lib, L):
     assert np.array_equal(got, want)
 
 
-def test_same_bits_across_the_scalar_ring_and_masks(cuda_lib):
+@pytest.mark.parametrize("L", [3, 4, 6, 7, 31, 33, 64, 65, 97, 129, 157, 160])
+def test_same_bits_under_the_delj_trick(cuda_lib, monkeypatch, L):
+    from dadi_gb300 import _lib, batch, integration
+    monkeypatch.setattr(integration, "use_delj_trick", True)
+    rec = batch.im_instances(_sets(3, 36 if L < 40 else 6, L))
+    rec["gamma"][0, 0, 1] = 8.0
+    if L == 160:  # beyond the delj trick's shared memory with one warp for both: refused
+        with pytest.raises(_lib.DgbError):
+            _both(L, rec)
+        return
+    got, want = _both(L, rec)
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("delj", [False, True])
+def test_same_bits_across_the_scalar_ring_and_masks(cuda_lib, monkeypatch, delj):
     """Schedules of 0 to 130 steps in one queue, frozen axes and suppressed
     mutations, selection."""
-    from dadi_gb300 import batch
+    from dadi_gb300 import batch, integration
+    monkeypatch.setattr(integration, "use_delj_trick", delj)
     p = _sets(24, 60, 1)
     p[:, 3] *= np.linspace(0, 2.2, 24)
     p[8:16, 4:] = 0
