@@ -32,6 +32,7 @@
 #include "dgb_cluster.cuh"
 #include "dgb_common.cuh"
 #include "dgb_internal.h"
+#include "dgb_split.cuh"
 
 namespace dgb {
 
@@ -677,6 +678,439 @@ __global__ void __launch_bounds__(AD_THREADS) k_adjoint2d(ADArgs A)
 }
 
 
+// ------------------------------- the trajectory-mode walk on groups of warps
+
+// k_adjoint2d<true> with its parts on their own warps.  The transposed solves
+// need the adjoint, their factors only the parameter rows, and a sweep's
+// contraction only its result and the stored trajectory; so in phase m
+//   group 0 solves sweep m, from one copy of the adjoint into another,
+//   group 1 forms the factors of sweep m + 1,
+//   groups 2 and 3 contract sweep m - 1 (the dt and nu sums; the m sum),
+//   group 4 forms the vectors and scalars to come, and the gamma and h sums
+//   of sweep m - 1 where a parameter depends on them,
+// one lane per line each, with one barrier per phase (sweeps go y, x of step
+// n - 1, then of n - 2, ...).  Each sum runs over a line's points in
+// k_adjoint2d's order and each line's lane adds up its steps in that order, so
+// the gradients are bitwise the same.  Grids whose two copies fit shared memory
+// (up to 112 points).
+constexpr int ADW_MAXWARPS = 4;
+constexpr int ADW_GROUPS = 5;
+
+struct ADWShared {
+    AxisScalars ax[2 * K2W_STEPS][2]; // ring over the steps walked
+    double inj[2 * K2W_STEPS], dinj_dt[2 * K2W_STEPS], dinj_th[2 * K2W_STEPS];
+    double red[ADW_MAXWARPS][NPAR];
+    int item;
+};
+
+// Doubles of shared memory: two adjoints, grid constants, the transposed and
+// the contraction vectors of both axes, the sums of groups 3 and 4 for the
+// two steps in flight.
+__host__ __device__ inline size_t adw_smem_doubles(int L)
+{
+    const int pitch = (L % 2) ? L : L + 1;
+    return 2 * (size_t)L * pitch + (6 + 10 + 8 + 4 * 2 + 8 * 2) * (size_t)L;
+}
+
+// Points of a line and of the stored densities along it, with the rows of the
+// next ADW_B points loaded ahead: f(i, mu_i, p_i, r_i, mu_{i+1}, p_{i+1}).
+constexpr int ADW_B = 4;
+
+template <bool RHS, typename F>
+__device__ __forceinline__ void adw_walk(const double *mu, int msp, const double *p,
+                                         const double *r, int sp, int L, F f)
+{
+    double mi = mu[0], pi = p[0];
+    double pn[ADW_B], rn[ADW_B];
+    auto load = [&](int i0) {
+#pragma unroll
+        for (int k = 0; k < ADW_B; k++) {
+            pn[k] = p[(size_t)min(i0 + k + 1, L - 1) * sp];
+            if (RHS)
+                rn[k] = r[(size_t)min(i0 + k, L - 1) * sp];
+        }
+    };
+    load(0);
+    for (int i0 = 0; i0 < L; i0 += ADW_B) {
+        double pv[ADW_B], rv[ADW_B];
+#pragma unroll
+        for (int k = 0; k < ADW_B; k++) {
+            pv[k] = pn[k];
+            rv[k] = RHS ? rn[k] : 0.0;
+        }
+        load(i0 + ADW_B);
+#pragma unroll
+        for (int k = 0; k < ADW_B; k++) {
+            const int i = i0 + k;
+            if (i >= L)
+                break;
+            const double mn = mu[min(i + 1, L - 1) * msp];
+            f(i, mi, pi, rv[k], mn, pv[k]);
+            mi = mn;
+            pi = pv[k];
+        }
+    }
+}
+
+template <int W>
+__global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs A)
+{
+    extern __shared__ __align__(16) double smem[];
+    __shared__ ADWShared S;
+    constexpr int ng = 32 * W;
+    const int tid = threadIdx.x, group = tid / ng, q = tid - group * ng;
+    const int pitch = (A.Lmax % 2) ? A.Lmax : A.Lmax + 1;
+    const size_t psz = (size_t)A.Lmax * pitch;
+    double *lam = smem; // copy b at lam + b * psz
+    GridVecs g;
+    double *p = smem + 2 * psz;
+    g.x = p; p += A.Lmax;
+    g.xv = p; p += A.Lmax;
+    g.dfac = p; p += A.Lmax;
+    g.xInt = p; p += A.Lmax;
+    g.ih = p; p += A.Lmax;
+    g.dx = p; p += A.Lmax;
+    double *tv = p; p += 10 * A.Lmax;   // transposed vectors, [axis][A1 A0 C1 C0 B0]
+    double *cvec = p; p += 8 * A.Lmax;  // contraction factors, [axis][P Q FG FH]
+    double *s3 = p; p += 8 * A.Lmax;    // group 3's sums, [step parity][axis][sm, bm][line]
+    double *s4 = p;                     // group 4's, [step parity][axis][sg, sh, bg, bh][line]
+    double *slice = A.scratch + (size_t)blockIdx.x * k2w_slice_doubles(A.Lmax, true);
+
+    for (;;) {
+        if (tid == 0)
+            S.item = atomicAdd(A.counter, 1);
+        __syncthreads();
+        const int w = S.item;
+        if (w >= A.nwork)
+            break;
+        const int wid = A.order[w];
+        const int inst = wid / A.ngrids, gi = wid - inst * A.ngrids;
+        const int L = A.L[gi], LP = k2w_pitch(L);
+        const size_t LL = (size_t)L * L, stride = (size_t)L * LP;
+        const double *xx = A.xx_all + A.xx_off[gi];
+        double *lam_g = A.lam + A.out_off[gi] + (size_t)inst * LL;
+        const int sidx = A.sched_per_grid ? wid : inst;
+        const double *rows = A.table + A.row_off[sidx] * 11;
+        const double *drows = A.drows + A.row_off[sidx] * NQ * NPAR;
+        const int n = A.row_cnt[sidx];
+        const int frozen = A.masks ? (A.masks[inst] & 0xff) : 0;
+        const int nomut = A.masks ? (A.masks[inst] >> 8 & 0xff) : 0;
+        const bool injx = !(frozen & 1) && !(nomut & 1), injy = !(frozen & 2) && !(nomut & 2);
+        const double *tphi = A.traj + A.traj_off[wid];
+        const double *tchi = tphi + (size_t)(n + 1) * LL;
+        for (int i = tid; i < L; i += blockDim.x) {
+            double x = xx[i];
+            g.x[i] = x;
+            g.xv[i] = x * (1. - x);
+            if (i < L - 1) {
+                double d = xx[i + 1] - x;
+                g.dx[i] = d;
+                g.ih[i] = 1.0 / (2 * d);
+                g.xInt[i] = 0.5 * (xx[i + 1] + x);
+            }
+        }
+        for (size_t idx = tid; idx < LL; idx += blockDim.x) {
+            const int r = (int)(idx / L), c = (int)(idx - (size_t)r * L);
+            lam[psz + r * pitch + c] = lam_g[idx]; // sweep 0 reads copy 1
+        }
+        __syncthreads();
+        for (int i = tid; i < L; i += blockDim.x) {
+            if (i == 0)
+                g.dfac[i] = 2. / g.dx[0];
+            else if (i == L - 1)
+                g.dfac[i] = 2. / g.dx[L - 2];
+            else
+                g.dfac[i] = 2. / (g.dx[i] + g.dx[i - 1]);
+        }
+        __syncthreads();
+        const int j0 = (g.x[0] == 0.0) ? 0 : -1;
+        const int j1 = (g.x[L - 1] == 1.0) ? L - 1 : -1;
+        const int nsw = 2 * n; // sweep m: axis 1 - (m & 1) of step n - 1 - (m >> 1)
+        auto tvecs = [&](int a) {
+            double *v = tv + (size_t)a * 5 * L;
+            AxisVecs t;
+            t.A1 = v;
+            t.A0 = v + L;
+            t.C1 = v + 2 * L;
+            t.C0 = v + 3 * L;
+            t.B0 = v + 4 * L;
+            t.G = t.Pv = t.Qv = t.VI = t.DF = nullptr;
+            return t;
+        };
+        // whether a parameter depends on gamma or h in step k (a whole warp)
+        auto selects = [&](int k) {
+            const int lane = tid & 31;
+            const double d = lane < 4 * NPAR ? drows[((size_t)k * NQ + Q_G0) * NPAR + lane] : 0.0;
+            return __any_sync(0xffffffffu, d != 0.0) != 0;
+        };
+        // the transposed vectors of sweep m (and, as they run out, the scalars
+        // of K2W_STEPS steps)
+        auto prepare = [&](int m) {
+            if (m >= nsw)
+                return;
+            const int a = 1 - (m & 1), st = m >> 1;
+            if (a == 1 && st % K2W_STEPS == 0) {
+                const int t = st + (q >> 1), b = t % (2 * K2W_STEPS);
+                const double *row = rows + (size_t)(n - 1 - t) * 11;
+                if (q < 2 * K2W_STEPS && t < n) {
+                    axis_scalars_2d(S.ax[b][q & 1], q & 1, row, g, L);
+                    if (!(q & 1)) {
+                        S.inj[b] = inject_value(2, row[0], row[1], g.x[0], g.x[1], g.x[2]);
+                        S.dinj_dt[b] = inject_value(2, 1.0, row[1], g.x[0], g.x[1], g.x[2]);
+                        S.dinj_th[b] = inject_value(2, row[0], 1.0, g.x[0], g.x[1], g.x[2]);
+                    }
+                }
+                bar_group(1, ng);
+            }
+            AxisVecs t = tvecs(a);
+            for (int i = q; i < L; i += ng) {
+                const AxisEntry e = axis_entry(i, L, g, S.ax[st % (2 * K2W_STEPS)][a], 1.0);
+                // row i's super- and subdiagonal become the next's sub-, the
+                // previous one's superdiagonal
+                t.B0[i] = e.B0;
+                if (i == 0)
+                    t.A1[i] = t.A0[i] = 0.0;
+                else
+                    t.C1[i - 1] = e.A1, t.C0[i - 1] = e.A0;
+                if (i == L - 1)
+                    t.C1[i] = t.C0[i] = 0.0;
+                else
+                    t.A1[i + 1] = e.C1, t.A0[i + 1] = e.C0;
+            }
+        };
+        auto factors = [&](int m) { // the contraction factors of sweep m
+            const int a = 1 - (m & 1);
+            const AxisScalars &s = S.ax[(m >> 1) % (2 * K2W_STEPS)][a];
+            double *c = cvec + (size_t)a * 4 * L;
+            for (int i = q; i < L - 1; i += ng) {
+                const double inu = s.inv_nu, hh = s.h, gam = s.gamma;
+                const double xi = g.xInt[i];
+                const double xx1 = xi * (1. - xi);
+                c[i] = inu * g.xv[i] * g.ih[i];
+                c[L + i] = inu * g.xv[i + 1] * g.ih[i];
+                c[2 * L + i] = 2 * (hh + (1. - 2 * hh) * xi) * xx1;
+                c[3 * L + i] = gam * 2 * (1. - 2 * xi) * xx1;
+            }
+        };
+        double acc[NPAR];
+#pragma unroll
+        for (int k = 0; k < NPAR; k++)
+            acc[k] = 0;
+        double smr[2] = {0, 0}, smp[2] = {0, 0}, snu[2] = {0, 0}, bnu[2] = {0, 0}, lin = 0;
+        if (group == 4) {
+            prepare(0);
+            prepare(1);
+        }
+        __syncthreads();
+        for (int m = -1; m <= nsw + 1; m++) {
+            if (group == 0) {
+                if (m >= 0 && m < nsw && q < L) {
+                    const int a = 1 - (m & 1);
+                    const size_t o = (size_t)q * ((a == 0) ? 1 : pitch);
+                    const int sp = (a == 0) ? pitch : 1;
+                    const double *src = lam + ((m + 1) & 1) * psz + o;
+                    double *dst = lam + (m & 1) * psz + o;
+                    if (frozen >> a & 1)
+                        for (int i = 0; i < L; i++)
+                            dst[i * sp] = src[i * sp];
+                    else
+                        k2w_solve<true>(src, dst, sp, L, tvecs(a), 0.0,
+                                        slice + (size_t)a * 3 * stride + q, stride, LP);
+                }
+            } else if (group == 1) {
+                const int f = m + 1, a = 1 - (f & 1);
+                if (f < nsw && !(frozen >> a & 1) && q < L) {
+                    const AxisScalars &s = S.ax[(f >> 1) % (2 * K2W_STEPS)][a];
+                    k2w_factor<true>(tvecs(a), s, L, s.mig[1 - a] * g.x[q],
+                                     (q == j0) ? s.bcs : 0.0, (q == j1) ? s.bce : 0.0,
+                                     slice + (size_t)a * 3 * stride + q, stride, LP);
+                }
+            } else {
+                if (group == 2 && m >= 3 && (m & 1)) {
+                    // every sum of the step whose x sweep was m - 2
+                    const int st = (m - 3) >> 1, k = n - 1 - st, b = st % (2 * K2W_STEPS);
+                    const bool sel = selects(k);
+                    if (q < L) {
+                        double G[NQ];
+#pragma unroll
+                        for (int i = 0; i < NQ; i++)
+                            G[i] = 0;
+                        for (int a = 1; a >= 0; a--) {
+                            if (frozen >> a & 1)
+                                continue;
+                            const double dt = S.ax[b][a].dt;
+                            const double *u3 = s3 + ((size_t)((st & 1) * 2 + a) * 2) * L + q;
+                            const double *u4 = s4 + ((size_t)((st & 1) * 2 + a) * 4) * L + q;
+                            G[Q_DT] -= (smr[a] - smp[a]) / dt;
+                            G[a ? Q_NU1 : Q_NU0] -= dt * snu[a] + bnu[a];
+                            G[a ? Q_M10 : Q_M01] -= dt * u3[0] + u3[L];
+                            if (sel) {
+                                G[a ? Q_G1 : Q_G0] -= dt * u4[0] + u4[2 * L];
+                                G[a ? Q_H1 : Q_H0] -= dt * u4[L] + u4[3 * L];
+                            }
+                        }
+                        if (q == 0) {
+                            G[Q_DT] += lin * S.dinj_dt[b];
+                            G[Q_TH] += lin * S.dinj_th[b];
+                        }
+                        const double *D = drows + (size_t)k * NQ * NPAR;
+#pragma unroll
+                        for (int j = 0; j < NPAR; j++) {
+                            double sacc = acc[j];
+#pragma unroll
+                            for (int i = 0; i < NQ; i++)
+                                if (sel || i < Q_G0 || i > Q_H1)
+                                    sacc = fma(G[i], D[i * NPAR + j], sacc);
+                            acc[j] = sacc;
+                        }
+                    }
+                }
+                const int c = m - 1, a = 1 - (c & 1), st = c >> 1, k = n - 1 - st;
+                if (c >= 0 && c < nsw) {
+                    const AxisScalars &s = S.ax[st % (2 * K2W_STEPS)][a];
+                    const bool live = q < L && !(frozen >> a & 1);
+                    const int msp = (a == 0) ? pitch : 1, sp = (a == 0) ? L : 1;
+                    const double *mu = lam + (c & 1) * psz + (size_t)q * ((a == 0) ? 1 : pitch);
+                    // y: phi_{k+1} and the right-hand side chi_k; x: chi_k and
+                    // phi_k with the injection
+                    const double *ph = (a == 0) ? tchi + (size_t)k * LL : tphi + (size_t)(k + 1) * LL;
+                    const double *rh = (a == 0) ? tphi + (size_t)k * LL : tchi + (size_t)k * LL;
+                    const double *pl = ph + (size_t)q * ((a == 0) ? 1 : L);
+                    const double *rl = rh + (size_t)q * ((a == 0) ? 1 : L);
+                    const double *cv = cvec + (size_t)a * 4 * L;
+                    const double dt = s.dt, inu = s.inv_nu, gam = s.gamma, hh = s.h;
+                    if (group == 2) {
+                        if (live) {
+                            double r0 = 0, r1 = 0, r2 = 0;
+                            const int ix = (a == 0 && injx && q == 0) ? 1 : -1;
+                            const int iy = (a == 0 && injy && q == 1) ? 0 : -1;
+                            const double inj = S.inj[st % (2 * K2W_STEPS)];
+                            adw_walk<true>(mu, msp, pl, rl, sp, L,
+                                           [&](int i, double mi, double pi, double ri, double mn,
+                                               double pn) {
+                                if (i == ix)
+                                    ri += inj;
+                                if (i == iy)
+                                    ri += inj;
+                                r0 = fma(mi, ri, r0);
+                                r1 = fma(mi, pi, r1);
+                                if (i < L - 1) {
+                                    const double Di = g.dfac[i] * mi - g.dfac[i + 1] * mn;
+                                    r2 = fma(Di, (cv[L + i] * pn - cv[i] * pi) * inu, r2);
+                                }
+                            });
+                            double bn = 0;
+                            if (q == j0 && s.bcs != 0.0) {
+                                double f = dt * 2. / g.dx[0], w = mu[0] * pl[0];
+                                bn += w * f * (-0.5 * inu * inu);
+                            }
+                            if (q == j1 && s.bce != 0.0) {
+                                double f = dt * 2. / g.dx[L - 2];
+                                double w = mu[(L - 1) * msp] * pl[(size_t)(L - 1) * sp];
+                                bn += w * f * (-0.5 * inu * inu);
+                            }
+                            smr[a] = r0;
+                            smp[a] = r1;
+                            snu[a] = r2;
+                            bnu[a] = bn;
+                        }
+                        if (a == 0 && q == 0) // the injected points, after the x solve
+                            lin = (injx ? mu[pitch] : 0.0) + (injy ? mu[1] : 0.0);
+                    } else if (group == 3) {
+                        if (live) {
+                            double r = 0, bm = 0;
+                            const double o = g.x[q];
+                            adw_walk<false>(mu, msp, pl, rl, sp, L,
+                                            [&](int i, double mi, double pi, double, double mn,
+                                                double pn) {
+                                if (i < L - 1) {
+                                    const double Di = g.dfac[i] * mi - g.dfac[i + 1] * mn;
+                                    const double hp = 0.5 * (pi + pn);
+                                    r = fma(Di * (o - g.xInt[i]), hp, r);
+                                }
+                            });
+                            if (q == j0 && s.bcs != 0.0) {
+                                double x0 = g.x[0], f = dt * 2. / g.dx[0], w = mu[0] * pl[0];
+                                bm += w * f * x0;
+                            }
+                            if (q == j1 && s.bce != 0.0) {
+                                double xl = g.x[L - 1], f = dt * 2. / g.dx[L - 2];
+                                double w = mu[(L - 1) * msp] * pl[(size_t)(L - 1) * sp];
+                                bm += w * f * (1. - xl);
+                            }
+                            double *u = s3 + ((size_t)((st & 1) * 2 + a) * 2) * L + q;
+                            u[0] = r;
+                            u[L] = bm;
+                        }
+                    } else if (selects(k)) {
+                        if (live) {
+                            double rg = 0, rh2 = 0, bg = 0, bh = 0;
+                            adw_walk<false>(mu, msp, pl, rl, sp, L,
+                                            [&](int i, double mi, double pi, double, double mn,
+                                                double pn) {
+                                if (i < L - 1) {
+                                    const double Di = g.dfac[i] * mi - g.dfac[i + 1] * mn;
+                                    const double hp = 0.5 * (pi + pn);
+                                    rg = fma(Di * cv[2 * L + i], hp, rg);
+                                    rh2 = fma(Di * cv[3 * L + i], hp, rh2);
+                                }
+                            });
+                            if (q == j0 && s.bcs != 0.0) {
+                                double x0 = g.x[0], f = dt * 2. / g.dx[0], w = mu[0] * pl[0];
+                                bg -= w * f * (2 * (hh + (1. - 2 * hh) * x0) * x0 * (1. - x0));
+                                bh -= w * f * (gam * 2 * (1. - 2 * x0) * x0 * (1. - x0));
+                            }
+                            if (q == j1 && s.bce != 0.0) {
+                                double xl = g.x[L - 1], f = dt * 2. / g.dx[L - 2];
+                                double w = mu[(L - 1) * msp] * pl[(size_t)(L - 1) * sp];
+                                bg += w * f * (2 * (hh + (1. - 2 * hh) * xl) * xl * (1. - xl));
+                                bh += w * f * (gam * 2 * (1. - 2 * xl) * xl * (1. - xl));
+                            }
+                            double *u = s4 + ((size_t)((st & 1) * 2 + a) * 4) * L + q;
+                            u[0] = rg;
+                            u[L] = rh2;
+                            u[2 * L] = bg;
+                            u[3 * L] = bh;
+                        }
+                    }
+                }
+                if (group == 4) {
+                    if (m >= 0 && m < nsw)
+                        factors(m);
+                    if (m >= 0)
+                        prepare(m + 2);
+                }
+            }
+            __syncthreads();
+        }
+        const double *fin = lam + ((nsw + 1) & 1) * psz; // the last sweep's copy
+        for (size_t idx = tid; idx < LL; idx += blockDim.x) {
+            // dJ/dphi_initial back to the caller's array
+            const int r = (int)(idx / L), c = (int)(idx - (size_t)r * L);
+            lam_g[idx] = fin[r * pitch + c];
+        }
+        // block reduction of acc into this work item's row of grad
+        if (group == 2) {
+#pragma unroll
+            for (int j = 0; j < NPAR; j++) {
+                double v = acc[j];
+                for (int off = 16; off > 0; off >>= 1)
+                    v += __shfl_down_sync(0xffffffffu, v, off);
+                if ((q & 31) == 0)
+                    S.red[q >> 5][j] = v;
+            }
+        }
+        __syncthreads();
+        if (tid < NPAR) {
+            double v = 0;
+            for (int wv = 0; wv < W; wv++)
+                v += S.red[wv][tid];
+            A.grad[((size_t)inst * A.ngrids + gi) * NPAR + tid] = v;
+        }
+        __syncthreads();
+    }
+}
+
 // Trajectory recomputation for the adjoint: one CTA per (work item,
 // checkpoint segment), all segments at once in a grid-stride loop, instead
 // of each work item's CTA recomputing its segments one after another before
@@ -1220,6 +1654,31 @@ static int adjoint2d_run(const int *masks, int ninst, const int *Ls, int ngrids,
         }
         return DGB_OK;
     }
+    if (traj) {
+        // factors, solves and contractions on their own warps where the
+        // adjoint's two copies fit and the workspace holds the factors of a
+        // CTA per SM (or per item)
+        const int warps = (Lmax + 31) / 32;
+        int dev = 0, optin = 0, nsm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        const size_t wsmem = adw_smem_doubles(Lmax) * sizeof(double);
+        const size_t slice = k2w_slice_doubles(Lmax, true) * sizeof(double);
+        long want = std::min<long>(nsm, nwalk);
+        if (max_blocks > 0)
+            want = std::min<long>(want, max_blocks);
+        if (warps <= ADW_MAXWARPS && wsmem + sizeof(ADWShared) + 1024 <= (size_t)optin &&
+            (long)((ws_bytes - 256) / slice) >= want) {
+            void (*const kernels[])(ADArgs) = {k_adjoint2d_ws<1>, k_adjoint2d_ws<2>,
+                                               k_adjoint2d_ws<3>, k_adjoint2d_ws<4>};
+            if (raise_smem_limit(kernels[warps - 1]))
+                return DGB_ERR_CUDA;
+            kernels[warps - 1]<<<(unsigned)want, 32 * warps * ADW_GROUPS, wsmem,
+                                 (cudaStream_t)stream>>>(A);
+            return cudaGetLastError() == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
+        }
+    }
     if (traj)
         k_adjoint2d<true><<<(unsigned)nblocks, AD_THREADS, smem, (cudaStream_t)stream>>>(A);
     else
@@ -1241,7 +1700,9 @@ extern "C" int dgb_adjoint2d(const int *masks, int ninst, const int *Ls, int ngr
 
 extern "C" size_t dgb_adjoint2d_traj_ws_bytes(int Lmax, int nblocks)
 {
-    return 256 + (size_t)nblocks * Lmax * Lmax * sizeof(double);
+    // Thomas scratch per CTA, or half the factors of k_adjoint2d_ws's (which
+    // runs one CTA per SM where this allows two)
+    return 256 + (size_t)nblocks * dgb::k2w_slice_doubles(Lmax, true) / 2 * sizeof(double);
 }
 
 extern "C" int dgb_adjoint2d_traj(const int *masks, int ninst, const int *Ls, int ngrids,
@@ -1280,6 +1741,8 @@ namespace dgb {
 int preload_adjoint2d()
 {
     return preload(k_sched2d_dual) + preload(k_adjoint2d<false>) + preload(k_adjoint2d<true>) +
-           preload(k_adjoint2d_traj) + preload(k_adjoint2d_cluster);
+           preload(k_adjoint2d_traj) + preload(k_adjoint2d_cluster) +
+           preload(k_adjoint2d_ws<1>) + preload(k_adjoint2d_ws<2>) +
+           preload(k_adjoint2d_ws<3>) + preload(k_adjoint2d_ws<4>);
 }
 } // namespace dgb

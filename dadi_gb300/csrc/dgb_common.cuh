@@ -472,55 +472,68 @@ __device__ __forceinline__ double vfunc_ref(double x, double nu, double beta)
     return v;
 }
 
-// Build entry i of the per-step vectors of one axis (called for i = 0..L-1
-// by different threads).  vscale multiplies V (the breeding-ratio factor of
-// Vfunc_beta in 1-D, 1 otherwise); beta1 is the breeding ratio itself for one
-// population and 0 otherwise (the delj path evaluates Vfunc_beta as written).
-__device__ __forceinline__ void build_axis_entry(int i, int L, const GridVecs &g,
-                                                 const AxisScalars &s, double vscale,
-                                                 bool delj, AxisVecs &v, double beta1 = 0.0)
+// Entry i of one axis for the default delta_j (see the header comment): the
+// affine coefficients of row i and its interior diagonal.  vscale multiplies V
+// (the breeding-ratio factor of Vfunc_beta in 1-D, 1 otherwise).
+struct AxisEntry {
+    double A1, A0, C1, C0, B0;
+};
+
+__device__ __forceinline__ AxisEntry axis_entry(int i, int L, const GridVecs &g,
+                                                const AxisScalars &s, double vscale)
 {
-    const double dt = s.dt;
     const double iv = s.inv_nu * vscale;
     auto Gk = [&](int k) { return msel(g.xInt[k], s.gamma, s.h) - s.msum * g.xInt[k]; };
-    double dfi = dt * g.dfac[i];
+    const double dfi = s.dt * g.dfac[i];
+    AxisEntry e = {0, 0, 0, 0, 0};
     double p_i = 0, q_im1 = 0;
     if (i < L - 1) {
         double G = Gk(i);
         double P = iv * g.xv[i] * g.ih[i];
         double Q = iv * g.xv[i + 1] * g.ih[i];
         p_i = fma(0.5, G, P);
-        v.C1[i] = 0.5 * dfi;
-        v.C0[i] = -dfi * fma(-0.5, G, Q);
-        if (delj) {
-            // the delj path rebuilds MInt per point in the reference order;
-            // per interval it needs the selection term, V[i]/(2 dx[i]),
-            // V[i+1]/(2 dx[i]) and VInt (dadi/integration2D.c:42-49,
-            // integration_shared.c:72-93), each rounded as the reference does
-            const double d2 = xm(2.0, g.dx[i]);
-            v.G[i] = msel_ref(g.xInt[i], s.gamma, s.h);
-            v.Pv[i] = xd(vfunc_ref(g.x[i], s.nu, beta1), d2);
-            v.Qv[i] = xd(vfunc_ref(g.x[i + 1], s.nu, beta1), d2);
-            v.VI[i] = vfunc_ref(g.xInt[i], s.nu, beta1);
-        }
-    } else {
-        v.C1[i] = 0;
-        v.C0[i] = 0;
+        e.C1 = 0.5 * dfi;
+        e.C0 = -dfi * fma(-0.5, G, Q);
     }
     if (i > 0) {
         double G = Gk(i - 1);
         double P = iv * g.xv[i - 1] * g.ih[i - 1];
         double Q = iv * g.xv[i] * g.ih[i - 1];
         q_im1 = fma(-0.5, G, Q);
-        v.A1[i] = -0.5 * dfi;
-        v.A0[i] = -dfi * fma(0.5, G, P);
-    } else {
-        v.A1[i] = 0;
-        v.A0[i] = 0;
+        e.A1 = -0.5 * dfi;
+        e.A0 = -dfi * fma(0.5, G, P);
     }
-    v.B0[i] = fma(dfi, p_i + q_im1, 1.0);
-    if (delj)
+    e.B0 = fma(dfi, p_i + q_im1, 1.0);
+    return e;
+}
+
+// Build entry i of the per-step vectors of one axis (called for i = 0..L-1
+// by different threads).  beta1 is the breeding ratio itself for one
+// population and 0 otherwise (the delj path evaluates Vfunc_beta as written).
+__device__ __forceinline__ void build_axis_entry(int i, int L, const GridVecs &g,
+                                                 const AxisScalars &s, double vscale,
+                                                 bool delj, AxisVecs &v, double beta1 = 0.0)
+{
+    const AxisEntry e = axis_entry(i, L, g, s, vscale);
+    v.A1[i] = e.A1;
+    v.A0[i] = e.A0;
+    v.C1[i] = e.C1;
+    v.C0[i] = e.C0;
+    v.B0[i] = e.B0;
+    if (delj) {
+        // the delj path rebuilds MInt per point in the reference order; per
+        // interval it needs the selection term, V[i]/(2 dx[i]),
+        // V[i+1]/(2 dx[i]) and VInt (dadi/integration2D.c:42-49,
+        // integration_shared.c:72-93), each rounded as the reference does
+        if (i < L - 1) {
+            const double d2 = xm(2.0, g.dx[i]);
+            v.G[i] = msel_ref(g.xInt[i], s.gamma, s.h);
+            v.Pv[i] = xd(vfunc_ref(g.x[i], s.nu, beta1), d2);
+            v.Qv[i] = xd(vfunc_ref(g.x[i + 1], s.nu, beta1), d2);
+            v.VI[i] = vfunc_ref(g.xInt[i], s.nu, beta1);
+        }
         v.DF[i] = g.dfac[i]; // unscaled: the delj rows are the reference's
+    }
 }
 
 // ------------------------------------------------------------ line solvers

@@ -75,3 +75,32 @@ def test_same_bits_where_the_solves_form_a_again(cuda_lib):
     from dadi_gb300 import batch
     got, want = _both(130, batch.im_instances(_sets(170, 6, 2)))
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("L", [3, 5, 31, 33, 64, 65, 97, 112, 113])
+@pytest.mark.parametrize("selection", [False, True])
+def test_adjoint_walk_on_groups_of_warps(cuda_lib, L, selection):
+    """The trajectory-mode backward walk (k_adjoint2d_ws up to 112 points)
+    against the segment-mode walk, which runs its parts one after the other:
+    the same bits, with and without parameters that gamma and h depend on,
+    frozen axes, schedules of none to more steps than the scalars' ring."""
+    import torch
+    from dadi_gb300 import batch
+    eng = batch.Batch2D((L,), (4, 4))
+    eng.cluster_adjoint, eng.cluster_forward = 0, False
+    p = _sets(6, 44 if L < 70 else 20, L)
+    p[0, 3] = 0.0
+    p[2:4, 4:] = 0
+    rec = batch.im_instances(p)
+    rec["gamma"][:, 0, 1], rec["h"][:, 1, 1] = 2.0, 0.3
+    rec["frozen"][2:4] = [1, 2]
+    rec["nomut"][4] = 1
+    seeds = batch.im_seeds(6)
+    if selection:
+        seeds["dform"][1:, 4, 0, 0] = 1.0   # gamma of population 1 moves with s
+        seeds["dform"][1:, 7, 0, 5] = -0.5  # h of population 2 with m21
+    data = torch.ones(5, 5, dtype=torch.float64, device="cuda")
+    got = [eng.loglik_and_grad(p, data, scale=10.0, rec=rec, seeds=seeds, trajectory=t)[1].cpu().numpy()
+           for t in (True, False)]
+    assert np.isfinite(got[1]).all() and np.abs(got[1]).max() > 0
+    assert np.array_equal(got[0], got[1])
