@@ -685,16 +685,17 @@ __global__ void __launch_bounds__(AD_THREADS) k_adjoint2d(ADArgs A)
 // contraction only its result and the stored trajectory; so in phase m
 //   group 0 solves sweep m, from one copy of the adjoint into another,
 //   group 1 forms the factors of sweep m + 1,
-//   groups 2 and 3 contract sweep m - 1 (the dt and nu sums; the m sum),
+//   groups 2, 3 and 5 contract sweep m - 1 (the dt sums; the m sum; the nu
+//   sum),
 //   group 4 forms the vectors and scalars to come, and the gamma and h sums
 //   of sweep m - 1 where a parameter depends on them,
 // one lane per line each, with one barrier per phase (sweeps go y, x of step
 // n - 1, then of n - 2, ...).  Each sum runs over a line's points in
 // k_adjoint2d's order and each line's lane adds up its steps in that order, so
 // the gradients are bitwise the same.  Grids whose two copies fit shared memory
-// (up to 112 points).
+// (up to 106 points).
 constexpr int ADW_MAXWARPS = 4;
-constexpr int ADW_GROUPS = 5;
+constexpr int ADW_GROUPS = 6;
 
 struct ADWShared {
     AxisScalars ax[2 * K2W_STEPS][2]; // ring over the steps walked
@@ -704,12 +705,12 @@ struct ADWShared {
 };
 
 // Doubles of shared memory: two adjoints, grid constants, the transposed and
-// the contraction vectors of both axes, the sums of groups 3 and 4 for the
+// the contraction vectors of both axes, the sums of groups 3, 5 and 4 for the
 // two steps in flight.
 __host__ __device__ inline size_t adw_smem_doubles(int L)
 {
     const int pitch = (L % 2) ? L : L + 1;
-    return 2 * (size_t)L * pitch + (6 + 10 + 8 + 4 * 2 + 8 * 2) * (size_t)L;
+    return 2 * (size_t)L * pitch + (6 + 10 + 8 + 8 * 2 + 8 * 2) * (size_t)L;
 }
 
 // Points of a line and of the stored densities along it, with the rows of the
@@ -752,6 +753,13 @@ __device__ __forceinline__ void adw_walk(const double *mu, int msp, const double
     }
 }
 
+// dfac_i mu_i - dfac_{i+1} mu_{i+1}, the second product rounded (off the FP64
+// pipe, as the other products here that are not part of a multiply-add).
+__device__ __forceinline__ double adw_diff(const GridVecs &g, int i, double mi, double mn)
+{
+    return fma(g.dfac[i], mi, -mul_full(mn, g.dfac[i + 1]));
+}
+
 template <int W>
 __global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs A)
 {
@@ -772,7 +780,7 @@ __global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs 
     g.dx = p; p += A.Lmax;
     double *tv = p; p += 10 * A.Lmax;   // transposed vectors, [axis][A1 A0 C1 C0 B0]
     double *cvec = p; p += 8 * A.Lmax;  // contraction factors, [axis][P Q FG FH]
-    double *s3 = p; p += 8 * A.Lmax;    // group 3's sums, [step parity][axis][sm, bm][line]
+    double *s3 = p; p += 16 * A.Lmax;   // groups 3, 5: [step parity][axis][sm, bm, snu, bnu][line]
     double *s4 = p;                     // group 4's, [step parity][axis][sg, sh, bg, bh][line]
     double *slice = A.scratch + (size_t)blockIdx.x * k2w_slice_doubles(A.Lmax, true);
 
@@ -896,7 +904,7 @@ __global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs 
 #pragma unroll
         for (int k = 0; k < NPAR; k++)
             acc[k] = 0;
-        double smr[2] = {0, 0}, smp[2] = {0, 0}, snu[2] = {0, 0}, bnu[2] = {0, 0}, lin = 0;
+        double smr[2] = {0, 0}, smp[2] = {0, 0}, lin = 0;
         if (group == 4) {
             prepare(0);
             prepare(1);
@@ -939,10 +947,10 @@ __global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs 
                             if (frozen >> a & 1)
                                 continue;
                             const double dt = S.ax[b][a].dt;
-                            const double *u3 = s3 + ((size_t)((st & 1) * 2 + a) * 2) * L + q;
+                            const double *u3 = s3 + ((size_t)((st & 1) * 2 + a) * 4) * L + q;
                             const double *u4 = s4 + ((size_t)((st & 1) * 2 + a) * 4) * L + q;
                             G[Q_DT] -= (smr[a] - smp[a]) / dt;
-                            G[a ? Q_NU1 : Q_NU0] -= dt * snu[a] + bnu[a];
+                            G[a ? Q_NU1 : Q_NU0] -= dt * u3[2 * L] + u3[3 * L];
                             G[a ? Q_M10 : Q_M01] -= dt * u3[0] + u3[L];
                             if (sel) {
                                 G[a ? Q_G1 : Q_G0] -= dt * u4[0] + u4[2 * L];
@@ -981,25 +989,37 @@ __global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs 
                     const double dt = s.dt, inu = s.inv_nu, gam = s.gamma, hh = s.h;
                     if (group == 2) {
                         if (live) {
-                            double r0 = 0, r1 = 0, r2 = 0;
+                            double r0 = 0, r1 = 0;
                             const int ix = (a == 0 && injx && q == 0) ? 1 : -1;
                             const int iy = (a == 0 && injy && q == 1) ? 0 : -1;
                             const double inj = S.inj[st % (2 * K2W_STEPS)];
                             adw_walk<true>(mu, msp, pl, rl, sp, L,
-                                           [&](int i, double mi, double pi, double ri, double mn,
-                                               double pn) {
+                                           [&](int i, double mi, double pi, double ri, double,
+                                               double) {
                                 if (i == ix)
                                     ri += inj;
                                 if (i == iy)
                                     ri += inj;
                                 r0 = fma(mi, ri, r0);
                                 r1 = fma(mi, pi, r1);
-                                if (i < L - 1) {
-                                    const double Di = g.dfac[i] * mi - g.dfac[i + 1] * mn;
-                                    r2 = fma(Di, (cv[L + i] * pn - cv[i] * pi) * inu, r2);
-                                }
                             });
-                            double bn = 0;
+                            smr[a] = r0;
+                            smp[a] = r1;
+                        }
+                        if (a == 0 && q == 0) // the injected points, after the x solve
+                            lin = (injx ? mu[pitch] : 0.0) + (injy ? mu[1] : 0.0);
+                    } else if (group == 5) {
+                        if (live) {
+                            double r = 0, bn = 0;
+                            adw_walk<false>(mu, msp, pl, rl, sp, L,
+                                            [&](int i, double mi, double pi, double, double mn,
+                                                double pn) {
+                                if (i < L - 1)
+                                    r = fma(adw_diff(g, i, mi, mn),
+                                            mul_full(fma(cv[L + i], pn, -mul_full(pi, cv[i])),
+                                                     inu),
+                                            r);
+                            });
                             if (q == j0 && s.bcs != 0.0) {
                                 double f = dt * 2. / g.dx[0], w = mu[0] * pl[0];
                                 bn += w * f * (-0.5 * inu * inu);
@@ -1009,13 +1029,10 @@ __global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs 
                                 double w = mu[(L - 1) * msp] * pl[(size_t)(L - 1) * sp];
                                 bn += w * f * (-0.5 * inu * inu);
                             }
-                            smr[a] = r0;
-                            smp[a] = r1;
-                            snu[a] = r2;
-                            bnu[a] = bn;
+                            double *u = s3 + ((size_t)((st & 1) * 2 + a) * 4 + 2) * L + q;
+                            u[0] = r;
+                            u[L] = bn;
                         }
-                        if (a == 0 && q == 0) // the injected points, after the x solve
-                            lin = (injx ? mu[pitch] : 0.0) + (injy ? mu[1] : 0.0);
                     } else if (group == 3) {
                         if (live) {
                             double r = 0, bm = 0;
@@ -1024,9 +1041,9 @@ __global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs 
                                             [&](int i, double mi, double pi, double, double mn,
                                                 double pn) {
                                 if (i < L - 1) {
-                                    const double Di = g.dfac[i] * mi - g.dfac[i + 1] * mn;
-                                    const double hp = 0.5 * (pi + pn);
-                                    r = fma(Di * (o - g.xInt[i]), hp, r);
+                                    const double Di = adw_diff(g, i, mi, mn);
+                                    const double hp = mul_full(pi + pn, 0.5);
+                                    r = fma(mul_full(Di, o - g.xInt[i]), hp, r);
                                 }
                             });
                             if (q == j0 && s.bcs != 0.0) {
@@ -1038,7 +1055,7 @@ __global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs 
                                 double w = mu[(L - 1) * msp] * pl[(size_t)(L - 1) * sp];
                                 bm += w * f * (1. - xl);
                             }
-                            double *u = s3 + ((size_t)((st & 1) * 2 + a) * 2) * L + q;
+                            double *u = s3 + ((size_t)((st & 1) * 2 + a) * 4) * L + q;
                             u[0] = r;
                             u[L] = bm;
                         }
@@ -1049,8 +1066,8 @@ __global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs 
                                             [&](int i, double mi, double pi, double, double mn,
                                                 double pn) {
                                 if (i < L - 1) {
-                                    const double Di = g.dfac[i] * mi - g.dfac[i + 1] * mn;
-                                    const double hp = 0.5 * (pi + pn);
+                                    const double Di = adw_diff(g, i, mi, mn);
+                                    const double hp = mul_full(pi + pn, 0.5);
                                     rg = fma(Di * cv[2 * L + i], hp, rg);
                                     rh2 = fma(Di * cv[3 * L + i], hp, rh2);
                                 }
