@@ -7,7 +7,23 @@
 
 namespace dgb {
 
-constexpr int ADN_MAXQ = 3 + 3 * DGB_MAX_DIM + DGB_MAX_DIM * (DGB_MAX_DIM - 1);
+// A line's contraction is summed in ADN_RUNS runs of intervals, and 32 lines
+// make one partial row.  The contraction is bound by one warp's FP64 issue
+// (13 instructions per interval, 64 cycles apart), so a tile is 32 lines with
+// ADN_RUNS threads each: one warp solves, four contract, and a lone grid of 40
+// points has 50 CTAs.  Against one thread per line on tiles of 64-128 lines, a
+// step backwards of the three-population growth model (two recomputing sweeps
+// and three of these) takes 163 us instead of 236 for one set at 40 points,
+// 173 instead of 237 for six, 298 instead of 394 for one at 80 points, 355
+// instead of 407 for four at 70, and 1749 instead of 1703 for 24 at 80.  Loads
+// of u and r four points ahead change nothing here.
+constexpr int ADN_RUNS = 4;
+
+inline long adn_rows(long nlines) { return (nlines + 31) / 32; }
+
+// This axis' entries of the row: dt, nu, gamma, h, then the migration rates
+// into it in ascending order.
+constexpr int ADN_NG = 4 + DGB_MAX_DIM - 1;
 
 struct ADNArgs {
     NDArgs nd;          // lam as nd.phi; axis, strides, table row
@@ -19,23 +35,60 @@ struct ADNArgs {
     long rec_off;       // offset of this integration's records after the grid constants
 };
 
-// Shared memory of an adjoint sweep CTA: the forward sweep's (tile, gam
-// unless it sits in a workspace slice, grid constants, vectors), the
-// transposed vectors and four per-interval contraction factors.
+// Shared memory of an adjoint sweep CTA of nt lines: the forward sweep's
+// (tile, gam unless it sits in a workspace slice, grid constants, vectors), the
+// transposed vectors and four per-interval contraction factors; at the end the
+// sums of the runs, in the same place.
 __host__ __device__ inline size_t adn_smem_doubles(int L, int nt, bool gsmem = true)
 {
-    return (size_t)L * (nt + 1) + (gsmem ? (size_t)L * nt : 0) + 20 * (size_t)L;
+    const size_t lines = (size_t)L * (nt + 1) + (gsmem ? (size_t)L * nt : 0) + 20 * (size_t)L;
+    const size_t sums = (size_t)(ADN_RUNS - 1) * ADN_NG * 32;
+    return lines > sums ? lines : sums;
 }
 
-// The transposed sweep and contraction of tile `tile_idx` (nt lines from
-// tile_idx * nt) of one integration: the body of k_adjoint_sweep_nd and of the
-// batched k_adjoint_sweep_batch.  Called by the whole CTA.
+// Whether an adjoint sweep takes lines of L points: what a tile of the forward
+// sweep's lines (nd_threads) would leave of shared memory decides, though
+// tiles of 32 lines need less.
+static bool adn_fits(int L, long nlines, bool gsmem)
+{
+    int dev = 0, optin = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
+            cudaSuccess)
+        return false;
+    return adn_smem_doubles(L, nd_threads(L, nlines), gsmem) * sizeof(double) +
+               sizeof(NDShared) + 2432 <=
+           (size_t)optin;
+}
+
+// Whether a launch over `tiles` tiles of 32 lines gives each line one thread,
+// which takes the runs in turn (the same sums in the same order), on tiles of
+// 128 lines: from eight tiles per SM on, if lines of 48 points or fewer let an
+// SM hold four such CTAs (16 solving warps, where 32-line tiles give six).
+// 32 sets at 40 points: 373 us a step backwards, 425 with ADN_RUNS threads;
+// on tiles of 64 lines 24 sets at 80 points take 1807 and 1794.
+static bool adn_wide(int L, long tiles)
+{
+    int dev = 0, sms = 152;
+    if (cudaGetDevice(&dev) == cudaSuccess)
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return L <= 48 && tiles >= 8L * sms;
+}
+
+// The transposed sweep and contraction of the 32 * WL lines from
+// tile_idx * 32 * WL of one integration, SG (1 or ADN_RUNS) threads per line:
+// the body of k_adjoint_sweep_nd and of the batched k_adjoint_sweep_batch.
+// Called by the whole CTA of 32 * WL * SG threads; red is shared.
+template <int WL, int SG>
 __device__ __forceinline__ void adn_tile(const ADNArgs &A, long tile_idx, double *smem,
-                                         NDShared &Sh, double (*red)[8],
+                                         NDShared &Sh, double (*red)[ADN_NG],
                                          double *gam_slice = nullptr)
 {
+    static_assert(SG == 1 || (SG == ADN_RUNS && WL == 1), "");
+    constexpr int nt = 32 * WL, bt = nt * SG;
     const NDArgs &N = A.nd;
-    const int nt = blockDim.x, L = N.L, P = N.ndim, ax = N.axis, tid = threadIdx.x;
+    const int L = N.L, P = N.ndim, ax = N.axis, tid = threadIdx.x;
+    const int ln = tid % nt, seg = tid / nt;
     const int stride = row_stride(P);
     double *tile, *gam;
     GridVecs g;
@@ -71,11 +124,11 @@ __device__ __forceinline__ void adn_tile(const ADNArgs &A, long tile_idx, double
                             ((size_t)(N.step - A.step0) * P + ax) * nd_rec_doubles(L, false);
         constexpr int NS = (int)(sizeof(AxisScalars) / sizeof(double));
         double *sp = reinterpret_cast<double *>(&Sh.s);
-        for (int i = tid; i < nd_grid_doubles(L); i += nt)
+        for (int i = tid; i < nd_grid_doubles(L); i += bt)
             g.x[i] = A.coef[i];
-        for (int i = tid; i < 5 * L; i += nt)
+        for (int i = tid; i < 5 * L; i += bt)
             v.A1[i] = rec[ND_HEAD + i];
-        for (int i = tid; i < ND_HEAD; i += nt) {
+        for (int i = tid; i < ND_HEAD; i += bt) {
             if (i < NS)
                 sp[i] = rec[i];
             else
@@ -86,11 +139,11 @@ __device__ __forceinline__ void adn_tile(const ADNArgs &A, long tile_idx, double
         if (tid == 0)
             nd_load_params(N, Sh, g);
         __syncthreads();
-        for (int i = tid; i < L; i += nt)
+        for (int i = tid; i < L; i += bt)
             build_axis_entry(i, L, g, Sh.s, Sh.vscale, false, v);
     }
     __syncthreads();
-    for (int i = tid; i < L; i += nt) {
+    for (int i = tid; i < L; i += bt) {
         vt.A1[i] = (i > 0) ? v.C1[i - 1] : 0.0;
         vt.A0[i] = (i > 0) ? v.C0[i - 1] : 0.0;
         vt.C1[i] = (i < L - 1) ? v.A1[i + 1] : 0.0;
@@ -115,15 +168,16 @@ __device__ __forceinline__ void adn_tile(const ADNArgs &A, long tile_idx, double
     const int j0 = (g.x[0] == 0.0) ? 0 : -1;
     const int j1 = (g.x[L - 1] == 1.0) ? L - 1 : -1;
     const AxisScalars &s = Sh.s;
-    double G[ADN_MAXQ];
-    for (int q = 0; q < stride; q++)
-        G[q] = 0;
-    if (tid < n) {
+    const int ng = 4 + P - 1;
+    double G[ADN_NG] = {};
+    const int tp = nt + 1;
+    long base = 0;
+    double W = 0, oo[DGB_MAX_DIM], bs = 0, be = 0;
+    int n1 = 0, k1 = -1;
+    if (ln < n) {
         int coord[DGB_MAX_DIM];
-        const long base = nd_line_base(N, l0 + tid, coord);
-        double W = 0, oo[DGB_MAX_DIM];
+        base = nd_line_base(N, l0 + ln, coord);
         bool all0 = true, all1 = true;
-        int n1 = 0, k1 = -1;
         for (int k = 0; k < P; k++) {
             oo[k] = g.x[coord[k]];
             if (k == ax)
@@ -140,88 +194,135 @@ __device__ __forceinline__ void adn_tile(const ADNArgs &A, long tile_idx, double
         }
         if (P == 1)
             all0 = all1 = true;
-        const double bs = all0 ? s.bcs : 0.0, be = all1 ? s.bce : 0.0;
-        const int tp = nt + 1;
+        bs = all0 ? s.bcs : 0.0;
+        be = all1 ? s.bce : 0.0;
         // mu = X^{-T} lambda on this line, in place in the tile
-        solve_line(tile + tid, tp, gam + tid, nt, L, W, bs, be, vt, s);
+        if (seg == 0)
+            solve_line(tile + ln, tp, gam + ln, nt, L, W, bs, be, vt, s);
+    }
+    __syncthreads();
+    if (ln < n) {
+        const double *mu = tile + ln;
         // contraction with u (forward output) and r (forward input)
-        const double *u = A.out + base, *r = A.rhs + base;
+        const double *u = A.out + base, *rhs = A.rhs + base;
         const long S = N.S;
         const double dt = s.dt, inu = s.inv_nu, gm = s.gamma, hh = s.h;
         const double inj0 = (n1 == 1 && k1 >= 0) ? Sh.inj[k1] : 0.0; // point 0 of this line
         const double inj1 = (n1 == 0) ? Sh.inj[ax] : 0.0;             // point 1 of this line
-        // the migration terms D_i (x_k - xInt_i) hp of every other population
-        // k from two sums: s1 = sum w, s2 = sum w xInt_i
-        double smr = 0, smp = 0, snu = 0, sg = 0, sh = 0, s1 = 0, s2 = 0;
-        double mi = tile[tid], ui = u[0];
-        double dmi = g.dfac[0] * mi;
-        for (int i = 0; i < L; i++) {
-            double ri = r[i * S];
-            if (i == 0)
-                ri += inj0;
-            if (i == 1)
-                ri += inj1;
-            smr = fma(mi, ri, smr);
-            smp = fma(mi, ui, smp);
-            if (i < L - 1) {
-                const double mn = tile[(i + 1) * tp + tid], un = u[(i + 1) * S];
-                const double dmn = g.dfac[i + 1] * mn;
-                const double Di = dmi - dmn;
-                const double w = Di * (ui + un);
-                snu = fma(Di, fma(-cP[i], ui, cQ[i] * un), snu);
-                s1 += w;
-                s2 = fma(w, g.xInt[i], s2);
-                sg = fma(w, gS[i], sg);
-                sh = fma(w, hS[i], sh);
-                mi = mn;
-                ui = un;
-                dmi = dmn;
+        // the corner terms, which few lines have (a branch of the warp's: FP64
+        // instructions switched off for a lane would cost the same)
+        double bnu = 0, bg = 0, bh = 0, bmf = 0, bml = 0;
+        if (seg == 0 && __any_sync(__activemask(), bs != 0.0 || be != 0.0)) {
+            if (bs != 0.0) {
+                const double x0 = g.x[0], f = dt * 2. / g.dx[0], w = mu[0] * u[0];
+                bnu += w * f * (-0.5 * inu * inu);
+                bmf = w * f * x0;
+                bg -= w * f * (2 * (hh + (1. - 2 * hh) * x0) * x0 * (1. - x0));
+                bh -= w * f * (gm * 2 * (1. - 2 * x0) * x0 * (1. - x0));
+            }
+            if (be != 0.0) {
+                const double xl = g.x[L - 1], f = dt * 2. / g.dx[L - 2];
+                const double w = mu[(L - 1) * tp] * u[(L - 1) * S];
+                bnu += w * f * (-0.5 * inu * inu);
+                bml = w * f * (1. - xl);
+                bg += w * f * (2 * (hh + (1. - 2 * hh) * xl) * xl * (1. - xl));
+                bh += w * f * (gm * 2 * (1. - 2 * xl) * xl * (1. - xl));
             }
         }
-        double sm[DGB_MAX_DIM];
-        for (int k = 0; k < P; k++)
-            sm[k] = 0.5 * fma(oo[k], s1, -s2);
-        double bnu = 0, bg = 0, bh = 0, bmf = 0, bml = 0;
-        if (bs != 0.0) {
-            const double x0 = g.x[0], f = dt * 2. / g.dx[0], w = tile[tid] * u[0];
-            bnu += w * f * (-0.5 * inu * inu);
-            bmf = w * f * x0;
-            bg -= w * f * (2 * (hh + (1. - 2 * hh) * x0) * x0 * (1. - x0));
-            bh -= w * f * (gm * 2 * (1. - 2 * x0) * x0 * (1. - x0));
+        const int run = (L + ADN_RUNS - 1) / ADN_RUNS;
+        for (int r0 = seg; r0 < ADN_RUNS; r0 += SG) {
+            // the migration terms D_i (x_k - xInt_i) hp of every other population
+            // k from two sums: s1 = sum w, s2 = sum w xInt_i
+            double smr = 0, smp = 0, snu = 0, sg = 0, sh = 0, s1 = 0, s2 = 0;
+            // the points [i0, i1) of the line, and the intervals from them
+            const int i0 = min(r0 * run, L), i1 = min(i0 + run, L), ib = min(i0, L - 1);
+            double mi = mu[ib * tp], ui = u[ib * S];
+            double dmi = g.dfac[ib] * mi;
+            for (int i = i0; i < i1; i++) {
+                double ri = rhs[i * S];
+                if (i == 0)
+                    ri += inj0;
+                if (i == 1)
+                    ri += inj1;
+                smr = fma(mi, ri, smr);
+                smp = fma(mi, ui, smp);
+                if (i < L - 1) {
+                    const double mn = mu[(i + 1) * tp], un = u[(i + 1) * S];
+                    const double dmn = g.dfac[i + 1] * mn;
+                    const double Di = dmi - dmn;
+                    const double w = Di * (ui + un);
+                    snu = fma(Di, fma(-cP[i], ui, cQ[i] * un), snu);
+                    s1 += w;
+                    s2 = fma(w, g.xInt[i], s2);
+                    sg = fma(w, gS[i], sg);
+                    sh = fma(w, hS[i], sh);
+                    mi = mn;
+                    ui = un;
+                    dmi = dmn;
+                }
+            }
+            const bool corner = r0 == 0;
+            double Q[ADN_NG] = {smp - smr, -fma(dt, snu, corner ? bnu : 0.0),
+                                -fma(dt, sg, corner ? bg : 0.0), -fma(dt, sh, corner ? bh : 0.0)};
+#pragma unroll
+            for (int k = 0; k < DGB_MAX_DIM; k++)
+                if (k < P && k != ax) {
+                    const double m = -fma(0.5 * dt, fma(oo[k], s1, -s2), corner ? bmf + bml : 0.0);
+#pragma unroll
+                    for (int e = 4; e < ADN_NG; e++)
+                        if (e == 4 + k - (k > ax))
+                            Q[e] = m;
+                }
+#pragma unroll
+            for (int q = 0; q < ADN_NG; q++)
+                G[q] = (SG > 1 || r0 == 0) ? Q[q] : G[q] + Q[q];
         }
-        if (be != 0.0) {
-            const double xl = g.x[L - 1], f = dt * 2. / g.dx[L - 2];
-            const double w = tile[(L - 1) * tp + tid] * u[(L - 1) * S];
-            bnu += w * f * (-0.5 * inu * inu);
-            bml = w * f * (1. - xl);
-            bg += w * f * (2 * (hh + (1. - 2 * hh) * xl) * xl * (1. - xl));
-            bh += w * f * (gm * 2 * (1. - 2 * xl) * xl * (1. - xl));
-        }
-        G[0] -= (smr - smp) / dt;
-        G[row_nu(P, ax)] -= dt * snu + bnu;
-        G[row_gamma(P, ax)] -= dt * sg + bg;
-        G[row_h(P, ax)] -= dt * sh + bh;
-        for (int k = 0; k < P; k++)
-            if (k != ax)
-                G[row_mig(P, ax, k)] -= dt * sm[k] + bmf + bml;
     }
-    __syncthreads();
     nd_tile_io(N, tile, nt, l0, n, true);
-    // fixed-order block reduction of G into this CTA's partial row
-    const int nw = nt >> 5;
-    for (int q = 0; q < stride; q++) {
+    // fixed-order sums of G: the runs of each line (in the tile's place), then
+    // the 32 lines of a warp
+    if (SG > 1) {
+        __syncthreads();
+        if (seg > 0)
+            for (int q = 0; q < ng; q++)
+                smem[((seg - 1) * ADN_NG + q) * nt + ln] = G[q];
+        __syncthreads();
+        if (seg > 0)
+            return;
+    }
+    const int lw = ln >> 5, lane = ln & 31;
+#pragma unroll
+    for (int q = 0; q < ADN_NG; q++) {
+        if (q >= ng)
+            break;
         double x = G[q];
+        for (int r = 0; r < SG - 1; r++)
+            x += smem[(r * ADN_NG + q) * nt + ln];
         for (int off = 16; off > 0; off >>= 1)
             x += __shfl_down_sync(0xffffffffu, x, off);
-        if ((tid & 31) == 0)
-            red[q][tid >> 5] = x;
+        if (lane == 0)
+            red[lw][q] = q ? x : x / s.dt;
     }
-    __syncthreads();
-    if (tid < stride) {
+    __syncwarp();
+    const long at = tile_idx * WL + lw;
+    if (at * 32 >= N.nlines)
+        return;
+    double *row = A.gpart + (size_t)at * stride;
+    for (int q = lane; q < stride; q += 32) {
         double x = 0;
-        for (int w = 0; w < nw; w++)
-            x += red[tid][w];
-        A.gpart[(size_t)tile_idx * stride + tid] = x;
+        if (q == 0)
+            x = red[lw][0];
+        else if (q == row_nu(P, ax))
+            x = red[lw][1];
+        else if (q == row_gamma(P, ax))
+            x = red[lw][2];
+        else if (q == row_h(P, ax))
+            x = red[lw][3];
+        else
+            for (int k = 0; k < P; k++)
+                if (k != ax && q == row_mig(P, ax, k))
+                    x = red[lw][4 + k - (k > ax)];
+        row[q] = x;
     }
 }
 

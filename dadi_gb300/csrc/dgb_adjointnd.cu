@@ -28,12 +28,13 @@
 
 namespace dgb {
 
-__global__ void k_adjoint_sweep_nd(ADNArgs A)
+template <int WL, int SG>
+__global__ void __launch_bounds__(32 * WL * SG) k_adjoint_sweep_nd(ADNArgs A)
 {
     extern __shared__ __align__(16) double smem[];
     __shared__ NDShared Sh;
-    __shared__ double red[ADN_MAXQ][8];
-    adn_tile(A, blockIdx.x, smem, Sh, red);
+    __shared__ double red[WL][ADN_NG];
+    adn_tile<WL, SG>(A, blockIdx.x, smem, Sh, red);
 }
 
 // Injection's part of dJ/d(dt) and dJ/d(theta0) for one step: lambda (the
@@ -45,16 +46,23 @@ __global__ void k_adjoint_inject_nd(const double *lam, const double *xx, const d
         adn_inject_terms(lam, xx, row, P, L, active, gout);
 }
 
+template <int WL, int SG>
+static int adn_launch_as(ADNArgs &A, cudaStream_t st)
+{
+    const size_t smem = adn_smem_doubles(A.nd.L, 32 * WL) * sizeof(double);
+    if (raise_smem_limit(k_adjoint_sweep_nd<WL, SG>))
+        return DGB_ERR_CUDA;
+    k_adjoint_sweep_nd<WL, SG>
+        <<<(unsigned)((adn_rows(A.nd.nlines) + WL - 1) / WL), 32 * WL * SG, smem, st>>>(A);
+    return cudaGetLastError() == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
+}
+
 static int adn_launch(ADNArgs &A, cudaStream_t st)
 {
-    const int L = A.nd.L;
-    int nt = nd_threads(L, A.nd.nlines);
-    size_t smem = adn_smem_doubles(L, nt) * sizeof(double);
-    long nblocks = (A.nd.nlines + nt - 1) / nt;
-    if (raise_smem_limit(k_adjoint_sweep_nd))
+    if (!adn_fits(A.nd.L, A.nd.nlines, true))
         return DGB_ERR_CUDA;
-    k_adjoint_sweep_nd<<<(unsigned)nblocks, nt, smem, st>>>(A);
-    return cudaGetLastError() == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
+    return adn_wide(A.nd.L, adn_rows(A.nd.nlines)) ? adn_launch_as<4, 1>(A, st)
+                                                   : adn_launch_as<1, ADN_RUNS>(A, st);
 }
 
 static void nd_set_axis(NDArgs &A, int ax)
@@ -115,12 +123,10 @@ extern "C" int dgb_integrate_table_states(double *phi, int ndim, int L, const do
 
 extern "C" size_t dgb_adjoint_table_nd_gpart_doubles(int ndim, int L)
 {
-    // per step: for each axis, one partial row per CTA of its sweep, plus the
+    // per step: for each axis, one partial row per 32 lines of its sweep, plus the
     // injection's two entries
     const long nlines = ipow(L, ndim - 1);
-    const int nt = nd_threads(L, nlines);
-    const long nb = (nlines + nt - 1) / nt;
-    return (size_t)ndim * nb * row_stride(ndim) + 2;
+    return (size_t)ndim * adn_rows(nlines) * row_stride(ndim) + 2;
 }
 
 extern "C" int dgb_adjoint_table_nd(double *lam, int ndim, int L, const double *xx,
@@ -143,7 +149,7 @@ extern "C" int dgb_adjoint_table_nd(double *lam, int ndim, int L, const double *
     const int active = ((1 << ndim) - 1) & ~frozen_mask & ~nomut_mask;
     const size_t per_step = dgb_adjoint_table_nd_gpart_doubles(ndim, L);
     const long nlines = ipow(L, ndim - 1);
-    const long nb = (nlines + nd_threads(L, nlines) - 1) / nd_threads(L, nlines);
+    const long nb = adn_rows(nlines);
     const int stride = row_stride(ndim);
     if (cudaMemsetAsync(gpart, 0, (size_t)nsteps * per_step * sizeof(double), st) !=
         cudaSuccess)
@@ -210,5 +216,9 @@ extern "C" int dgb_adjoint_table_nd(double *lam, int ndim, int L, const double *
 }
 
 namespace dgb {
-int preload_adjointnd() { return preload(k_adjoint_sweep_nd) + preload(k_adjoint_inject_nd); }
+int preload_adjointnd()
+{
+    return preload(k_adjoint_sweep_nd<1, ADN_RUNS>) + preload(k_adjoint_sweep_nd<4, 1>) +
+           preload(k_adjoint_inject_nd);
+}
 } // namespace dgb

@@ -863,11 +863,12 @@ struct ADNBatch {
 // every running integration: CTA b handles tile b % bpi of item b / bpi,
 // the per-line work of k_adjoint_sweep_nd on that item's lambda, recorded
 // and recomputed densities, records and partial rows.
-__global__ void k_adjoint_sweep_batch(ADNBatch B)
+template <int WL, int SG>
+__global__ void __launch_bounds__(32 * WL * SG) k_adjoint_sweep_batch(ADNBatch B)
 {
     extern __shared__ __align__(16) double smem[];
     __shared__ NDShared Sh;
-    __shared__ double red[ADN_MAXQ][8];
+    __shared__ double red[WL][ADN_NG];
     const long it = blockIdx.x / B.bpi;
     const long tl = blockIdx.x - it * B.bpi;
     const dgb_itemnd_adj I = B.items[it];
@@ -888,8 +889,8 @@ __global__ void k_adjoint_sweep_batch(ADNBatch B)
         j += !(frozen >> a & 1);
     A.gpart = B.gpart_all + I.gpart_off + k * B.per_step + (long)j * B.nb * row_stride(P);
     A.rec_off = it * B.item_coef;
-    adn_tile(A, tl, smem, Sh, red,
-             B.gam + (size_t)blockIdx.x * B.a.nd.L * blockDim.x);
+    adn_tile<WL, SG>(A, tl, smem, Sh, red,
+                     B.gam + (size_t)blockIdx.x * B.a.nd.L * (32 * WL));
 }
 
 // The injection's terms of step k, one thread per running item.
@@ -915,7 +916,7 @@ __global__ void k_adjoint_inject_batch(const dgb_itemnd_adj *items, int nact,
 // forward and for each recomputed axis).
 struct AdjLayout {
     BatchPlan p;
-    int nt, nb; // the transposed sweeps' lines per CTA and CTAs per item
+    int nb; // the transposed sweeps' partial rows per item
     size_t coef, gam, slots, gam_adj, items_adj, items_nd, total; // offsets in bytes
 };
 
@@ -934,10 +935,9 @@ static int adj_layout(int ndim, int L, int nitems, const dgb_settings *settings,
     w.gam = up(w.p.coef_doubles * sizeof(double));
     w.slots = w.gam + up(w.p.gam_doubles * sizeof(double));
     const long nlines = ipow(L, ndim - 1);
-    w.nt = nd_threads(L, nlines);
-    w.nb = (int)((nlines + w.nt - 1) / w.nt);
+    w.nb = (int)adn_rows(nlines);
     w.gam_adj = w.slots + up((size_t)nitems * (ndim > 1 ? ndim - 1 : 0) * N * sizeof(double));
-    w.items_adj = w.gam_adj + up((size_t)nitems * w.nb * w.nt * L * sizeof(double));
+    w.items_adj = w.gam_adj + up((size_t)nitems * ((w.nb + 3) / 4 * 4) * 32 * L * sizeof(double));
     w.items_nd = w.items_adj + up((size_t)nitems * sizeof(dgb_itemnd_adj));
     w.total = w.items_nd + up((size_t)(ndim + 1) * nitems * sizeof(dgb_itemnd));
     return DGB_OK;
@@ -1083,7 +1083,7 @@ extern "C" int dgb_batchnd_adjoint(const dgb_itemnd_adj *items, int nitems, int 
         return DGB_ERR_CUDA;
     // the transposed sweeps: the tiles of dgb_adjoint_table_nd, with the
     // Thomas scratch in workspace slices (twice the CTAs per SM)
-    const int nt = w.nt, nb = w.nb;
+    const int nb = w.nb;
     ADNBatch AB = {};
     nd_fill(AB.a.nd, nullptr, ndim, L, 0, xx);
     AB.a.nd.table = table;
@@ -1098,10 +1098,10 @@ extern "C" int dgb_batchnd_adjoint(const dgb_itemnd_adj *items, int nitems, int 
     AB.slot_stride = slot_stride;
     AB.item_coef = B.item_coef;
     AB.per_step = per_step;
-    AB.bpi = nb;
     AB.nb = nb;
-    const size_t asmem = adn_smem_doubles(L, nt, false) * sizeof(double);
-    if (raise_smem_limit(k_adjoint_sweep_batch))
+    if (!adn_fits(L, ipow(L, ndim - 1), false) ||
+        raise_smem_limit(k_adjoint_sweep_batch<1, ADN_RUNS>) ||
+        raise_smem_limit(k_adjoint_sweep_batch<4, 1>))
         return DGB_ERR_CUDA;
     const long inj_at = (long)ndim * nb * row_stride(ndim);
     const unsigned cpx = (unsigned)std::min<long>((N + 255) / 256, 64);
@@ -1138,7 +1138,14 @@ extern "C" int dgb_batchnd_adjoint(const dgb_itemnd_adj *items, int nitems, int 
             AB.a.nd.S = ipow(L, ndim - 1 - ax);
             AB.a.nd.LS = AB.a.nd.S * L;
             AB.a.nd.step = k;
-            k_adjoint_sweep_batch<<<(unsigned)(nact * nb), nt, asmem, st>>>(AB);
+            const int wl = adn_wide(L, nact * nb) ? 4 : 1;
+            AB.bpi = (nb + wl - 1) / wl;
+            const unsigned ctas = (unsigned)(nact * AB.bpi);
+            const size_t smem = adn_smem_doubles(L, 32 * wl, false) * sizeof(double);
+            if (wl == 1)
+                k_adjoint_sweep_batch<1, ADN_RUNS><<<ctas, 32 * ADN_RUNS, smem, st>>>(AB);
+            else
+                k_adjoint_sweep_batch<4, 1><<<ctas, 128, smem, st>>>(AB);
             if (cudaGetLastError() != cudaSuccess)
                 return DGB_ERR_CUDA;
         }
@@ -1485,7 +1492,8 @@ int preload_batchnd()
            preload(k_sweep_batch<true, false>) + preload(k_sweep_batch<true, true>) +
            preload(k_sweep_batch_pcr) + preload(k_sweep_batch_part<2>) +
            preload(k_sweep_batch_part<4>) + preload(k_sweep_batch_part<8>) +
-           preload(k_store_states) + preload(k_slot_copy) + preload(k_adjoint_sweep_batch) +
+           preload(k_store_states) + preload(k_slot_copy) + preload(k_adjoint_sweep_batch<1, ADN_RUNS>) +
+           preload(k_adjoint_sweep_batch<4, 1>) +
            preload(k_adjoint_inject_batch);
 }
 } // namespace dgb

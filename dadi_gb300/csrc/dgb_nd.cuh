@@ -234,12 +234,14 @@ __device__ __forceinline__ void nd_tile_io(const NDArgs &A, double *tile, int nt
             }
         }
     } else {
-        int t = threadIdx.x;
+        // one thread per line, or blockDim.x / nt of them (alternate points)
+        const int q = (int)threadIdx.x / nt, nq = (int)blockDim.x / nt;
+        const int t = (int)threadIdx.x - q * nt;
         if (t < n) {
             long line = l0 + t;
             long outer = line / A.S, inner = line - outer * A.S;
             double *g0 = A.phi + outer * A.LS + inner;
-            for (int p = 0; p < L; p++) {
+            for (int p = q; p < L; p += nq) {
                 if (store)
                     g0[p * A.S] = tile[p * tp + t];
                 else

@@ -386,7 +386,7 @@ int dgb_batch2d_count_steps(const dgb_inst2d *insts, int ninst,
  * and dJ/dphi_initial on exit; gpart (device,
  * nsteps x dgb_adjoint_table_nd_gpart_doubles) receives per step the partial
  * sums of dJ/d(table row entries): for each swept axis j (in sweep order)
- * one DGB_ROW_STRIDE(ndim) row per CTA of that sweep, followed by two
+ * one DGB_ROW_STRIDE(ndim) row per 32 lines of that sweep, followed by two
  * doubles, the injection's dJ/d(dt) and dJ/d(theta0).  Summing a step's
  * rows (any fixed order) and adding those two to entries 0 and 1 gives
  * dJ/d(row) for that step.  ws: (active axes - 1) x L^ndim doubles, and

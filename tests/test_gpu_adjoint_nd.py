@@ -131,6 +131,82 @@ def test_adjoint_records_match_inline_setup(cuda_lib, P, L, frozen):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("P,L", [(1, 3), (1, 34), (2, 3), (2, 5), (2, 31), (2, 33), (3, 6),
+                                 (3, 9), (4, 5)])
+def test_row_gradients_at_tile_and_run_edges(cuda_lib, P, L):
+    """dJ/d(table row), J = <w, phi after two steps>, against Richardson
+    central differences of the recorded forward, at line counts around one
+    tile of 32 and line lengths the four runs of a contraction do not divide.
+    Differences of 1e-3 and 5e-4 leave a truncation of (1e-3)^4 and a rounding
+    below 1e-11 of sum |w phi|, against a bar of GRAD_TOL of the entry's
+    gradient or of 1e-4 of that sum."""
+    import torch
+    from dadi_gb300 import _lib, integration
+    import cases
+    from util import table_rows
+    lib = cuda_lib
+    N, tab = L ** P, table_rows(P, 2, seed=11 * P + L)
+    tab[:, 2 + 3 * P] = 1.0  # beta, not differentiated
+    d_xx = torch.from_numpy(cases.grid("default", L)).cuda()
+    phi0 = np.abs(cases.initial_phi(5, (L,) * P)) + 1e-3
+    w = cases.initial_phi(6, (L,) * P) - 0.5
+    sh = _lib.stream_handle(torch)
+    ws, nws = _lib.workspace(torch, max(lib.dgb_workspace_bytes(0, P, L, 0),
+                                        lib.dgb_workspace_bytes(4, P, L, 0)))
+
+    def forward(t):
+        d_phi, d_tab = torch.from_numpy(phi0.copy()).cuda(), torch.from_numpy(t).cuda()
+        states = torch.empty(3 * N, dtype=torch.float64, device="cuda")
+        _lib.check(lib.dgb_integrate_table_states(
+            _lib.dptr(d_phi), P, L, _lib.dptr(d_xx), _lib.dptr(d_tab), 2, 0, 0,
+            _lib.dptr(states), _lib.dptr(ws), nws, sh), "dgb_integrate_table_states")
+        return states, d_tab, float(np.dot(w.ravel(), states[2 * N:].cpu().numpy()))
+
+    states, d_tab, _ = forward(tab)
+    J = float(np.dot(np.abs(w.ravel()), np.abs(states[2 * N:].cpu().numpy())))
+    per, stride = lib.dgb_adjoint_table_nd_gpart_doubles(P, L), integration.row_stride(P)
+    lam = torch.from_numpy(w.copy()).cuda()
+    gpart = torch.empty(2 * per, dtype=torch.float64, device="cuda")
+    _lib.check(lib.dgb_adjoint_table_nd(
+        _lib.dptr(lam), P, L, _lib.dptr(d_xx), _lib.dptr(d_tab), 2, 0, 0, _lib.dptr(states),
+        _lib.dptr(gpart), _lib.dptr(ws), nws, sh), "dgb_adjoint_table_nd")
+    gp = gpart.cpu().numpy().reshape(2, per)
+    G = gp[:, :per - 2].reshape(2, -1, stride).sum(axis=1)
+    G[:, :2] += gp[:, per - 2:]
+    for q in range(stride):
+        if q == 2 + 3 * P:
+            continue
+        D = np.zeros((2, 2))
+        for k in range(2):
+            for e, eps in enumerate((1e-3, 5e-4)):
+                h = eps * (tab[k, 0] if q == 0 else max(abs(tab[k, q]), 0.1))
+                up, dn = tab.copy(), tab.copy()
+                up[k, q] += h
+                dn[k, q] -= h
+                D[e, k] = (forward(up)[2] - forward(dn)[2]) / (2 * h)
+        fd = (4 * D[1] - D[0]) / 3
+        bar = GRAD_TOL * max(np.max(np.abs(fd)), 1e-4 * J)
+        assert np.max(np.abs(G[:, q] - fd)) <= bar, (q, G[:, q], fd)
+
+
+@pytest.mark.parametrize("L,n", [(10, 410), (47, 18)])
+def test_one_thread_per_line_gives_the_split_sums(cuda_lib, L, n):
+    """Batches with lines enough to fill the GPU (one thread per line on ragged
+    tiles of 128 lines) give each set's own gradient, which a few lines compute with four threads
+    each, bitwise."""
+    from dadi_gb300 import adjoint_nd
+    model = adjoint_nd.Growth3((L,), (4, 4, 4))
+    th = _theta()
+    th[9] = 0.004
+    sets = [th * (1 + 0.01 * (k % 7)) for k in range(n)]
+    data = np.ones((5, 5, 5))
+    many = model.loglik_and_grad_batch(sets, data, 10.0)
+    for k in (0, 3, n - 1):
+        ll, g, _ = model.loglik_and_grad(sets[k], data, 10.0)
+        assert float(ll) == float(many[k][0])
+        assert np.array_equal(g.cpu().numpy(), many[k][1].cpu().numpy())
+
+
 @pytest.mark.parametrize("P,L,frozen", [(3, 12, [0, 0, 0, 0]), (3, 14, [0, 4, 0, 1]),
                                         (4, 7, [0, 0, 2, 0]), (2, 20, [0, 1, 0, 0]),
                                         (1, 30, [0, 0, 0, 0])])
