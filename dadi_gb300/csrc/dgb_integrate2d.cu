@@ -20,8 +20,9 @@
 // longest-first from an atomic counter (one launch over all grids, or one
 // per grid size with a CTA shaped for it), or one CTA per item.  Under the
 // default delta_j the factorisations of a sweep run on other warps than its
-// solves (k_integrate2d_ws); k_integrate2d, one warp for both, serves the delj
-// trick, an explicit CTA size or scratch placement, and callers without
+// solves (k_integrate2d_ws), under the delj trick its coefficients
+// (k_integrate2d_delj); k_integrate2d, one warp for both, serves an explicit
+// CTA size or scratch placement, grids beyond 160 points, and callers without
 // workspace.
 //
 // Reference: the time loop of Integration.two_pops (dadi/Integration.py:

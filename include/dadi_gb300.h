@@ -75,8 +75,10 @@ typedef struct {
                                     largest grid for the solves and as many for the factors
                                     of the next sweep -- or 64 / 96 / 128 threads per CTA,
                                     one lane for both, where that many threads hold every
-                                    line (else the fewest warps, 2-4, that do); the delj
-                                    trick and gam_placement 1 always take the latter */
+                                    line (else the fewest warps, 2-4, that do);
+                                    gam_placement 1 always takes the latter.  Under the
+                                    delj trick the automatic choice forms each sweep's
+                                    coefficients ahead on further warps */
     int line_solver;             /* batched N-dimensional engine: 0 Thomas, one line per
                                     thread (dadi/tridiag.c:14-34); 1 parallel cyclic
                                     reduction, one warp per line (L <= 128); 2 partitioned
