@@ -1366,7 +1366,7 @@ __global__ void __launch_bounds__(AC_THREADS) k_adjoint2d_cluster(ADArgs A)
         // ---- y: mu = Y^{-T} lambda on the CTA's rows, contracted with
         // phi_{k+1} (the sweep's output) and chi_k (its input)
         if (!(frozen & 2)) {
-            c2_sweep_y(blk, pitch, L, R0, m, al, ga, yr, V.t[1], S.ax[1], g, j0, j1);
+            c2_sweep_y<true>(blk, pitch, L, R0, m, al, ga, yr, V.t[1], S.ax[1], g, j0, j1);
             const int p = tid % C2_ROWS, q = tid / C2_ROWS;
             if (p < m) {
                 const int mlen = L / C2_YSEG, extra = L % C2_YSEG;
@@ -1423,7 +1423,7 @@ __global__ void __launch_bounds__(AC_THREADS) k_adjoint2d_cluster(ADArgs A)
         // ---- x: nu = X^{-T} mu across the cluster, contracted with chi_k
         // (the sweep's output) and psi_k (its input)
         if (!(frozen & 1)) {
-            c2_sweep_x(cluster, NS, rank, blk, pitch, L, R0, m, al, ga, xr, zin, V.t[0],
+            c2_sweep_x<true>(cluster, NS, rank, blk, pitch, L, R0, m, al, ga, xr, zin, V.t[0],
                        S.ax[0], g, j0, j1);
             for (int j = tid; j < L; j += AC_THREADS)
                 hx[j] = blk[j];

@@ -23,6 +23,11 @@
 // every CTA of the cluster): they contain the barriers.  Further threads of
 // the CTA pass the two cluster barriers of c2_sweep_x on their own.  Default
 // delta_j rows only.
+//
+// FP64: the pivots on the FP64 pipe, and no further threads.  The forward
+// integration is faster on the integer pipes (19,546 steps of the three grids
+// 100, 110, 120: 0.67 s against 0.73), the adjoint's walk, whose code is three
+// times as long, on the FP64 pipe (1.46 s against 1.50); the bits are the same.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -37,6 +42,40 @@ constexpr int C2_YSEG = 8;  // segments per row in the y sweep
 constexpr int C2_XROW = 6;  // exported values per column: A' C' D' al ga de
 constexpr int C2_YSLOT = 8; // per (row, segment): A' C' D', al ga de / z row, z
 
+template <bool FP64>
+__device__ __forceinline__ void c2_pivot3(double bet, double t, double c, double d, double &u,
+                                          double &g, double &w)
+{
+    if (FP64) {
+        const double inv = rcp_newton_here(bet);
+        u = t * inv;
+        g = c * inv;
+        w = d * inv;
+    } else {
+        pivot3(bet, t, c, d, u, g, w);
+    }
+}
+
+template <bool FP64>
+__device__ __forceinline__ void c2_pivot(double bet, double t, double c, double &u, double &g)
+{
+    if (FP64) {
+        const double inv = rcp_newton_here(bet);
+        u = t * inv;
+        g = c * inv;
+    } else {
+        pivot(bet, t, c, u, g);
+    }
+}
+
+template <bool FP64> __device__ __forceinline__ void c2_bar()
+{
+    if (FP64)
+        __syncthreads();
+    else
+        bar_group(C2_BAR, C2_THREADS);
+}
+
 __host__ __device__ inline int c2_pitch(int L) { return (L % 2) ? L : L + 1; }
 
 // Rows of CTA r of S over L points: [*r0, *r0 + *m).
@@ -49,6 +88,7 @@ __host__ __device__ inline void c2_rows(int L, int S, int r, int *r0, int *m)
 
 // The x sweep of the CTA's rows; al, ga: C2_ROWS x L scratch ([p][j]); xr:
 // C2_XROW x L doubles read by the other CTAs; zin: 2 L doubles they write.
+template <bool FP64>
 __device__ __forceinline__ void c2_sweep_x(cooperative_groups::cluster_group &cluster, int S,
                                            int rank, double *blk, int pitch, int L, int R0,
                                            int m, double *al, double *ga, double *xr,
@@ -71,13 +111,13 @@ __device__ __forceinline__ void c2_sweep_x(cooperative_groups::cluster_group &cl
         int p = 1;
         double aa = arow(R0 + p);
         double alp, gap, dep;
-        pivot3(brow(R0 + p), aa, crow(R0 + p), blk[p * pitch + j], alp, gap, dep);
+        c2_pivot3<FP64>(brow(R0 + p), aa, crow(R0 + p), blk[p * pitch + j], alp, gap, dep);
         al[p * L + j] = alp;
         ga[p * L + j] = gap;
         blk[p * pitch + j] = dep;
         for (p = 2; p < m; p++) {
             aa = arow(R0 + p);
-            pivot3(fma(-aa, gap, brow(R0 + p)), -aa * alp, crow(R0 + p),
+            c2_pivot3<FP64>(fma(-aa, gap, brow(R0 + p)), -aa * alp, crow(R0 + p),
                    fma(-aa, dep, blk[p * pitch + j]), alp, gap, dep);
             al[p * L + j] = alp;
             ga[p * L + j] = gap;
@@ -99,7 +139,7 @@ __device__ __forceinline__ void c2_sweep_x(cooperative_groups::cluster_group &cl
         }
         const double c0 = crow(R0);
         double xa, xc, xd;
-        pivot3(fma(-c0, alu, brow(R0)), arow(R0), -c0 * gau, fma(-c0, deu, blk[j]), xa, xc, xd);
+        c2_pivot3<FP64>(fma(-c0, alu, brow(R0)), arow(R0), -c0 * gau, fma(-c0, deu, blk[j]), xa, xc, xd);
         xr[0 * L + j] = xa;
         xr[1 * L + j] = xc;
         xr[2 * L + j] = xd;
@@ -125,7 +165,7 @@ __device__ __forceinline__ void c2_sweep_x(cooperative_groups::cluster_group &cl
             const double rc = -gaq * Cn;
             const double rd = fma(-gaq, Dn, fma(-alq, Dp, deq));
             const double bet = (q == 0) ? rb : fma(-ra, gq, rb);
-            pivot(bet, (q == 0) ? rd : fma(-ra, u, rd), rc, u, gq);
+            c2_pivot<FP64>(bet, (q == 0) ? rd : fma(-ra, u, rd), rc, u, gq);
             gm[q] = gq;
             z[q] = u;
         }
@@ -147,11 +187,12 @@ __device__ __forceinline__ void c2_sweep_x(cooperative_groups::cluster_group &cl
             blk[p * pitch + j] =
                 fma(-ga[p * L + j], xl, fma(-al[p * L + j], xf, blk[p * pitch + j]));
     }
-    bar_group(C2_BAR, C2_THREADS);
+    c2_bar<FP64>();
 }
 
 // The y sweep of the CTA's rows; al, ga: L x C2_ROWS scratch ([c][p]); yr:
 // C2_YSLOT x C2_YSEG x C2_ROWS doubles of the segments' systems.
+template <bool FP64>
 __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0, int m,
                                            double *al, double *ga, double *yr,
                                            const AxisVecs &vv, const AxisScalars &s,
@@ -180,13 +221,13 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
         int c = s0 + 1;
         double aa = arow(c);
         double alp, gap, dep;
-        pivot3(brow(c), aa, crow(c), ph[c], alp, gap, dep);
+        c2_pivot3<FP64>(brow(c), aa, crow(c), ph[c], alp, gap, dep);
         al[c * C2_ROWS + p] = alp;
         ga[c * C2_ROWS + p] = gap;
         ph[c] = dep;
         for (c = s0 + 2; c < s0 + ml; c++) {
             aa = arow(c);
-            pivot3(fma(-aa, gap, brow(c)), -aa * alp, crow(c), fma(-aa, dep, ph[c]), alp, gap,
+            c2_pivot3<FP64>(fma(-aa, gap, brow(c)), -aa * alp, crow(c), fma(-aa, dep, ph[c]), alp, gap,
                    dep);
             al[c * C2_ROWS + p] = alp;
             ga[c * C2_ROWS + p] = gap;
@@ -208,12 +249,12 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
         }
         const double c0 = crow(s0);
         double xa, xc, xd;
-        pivot3(fma(-c0, alu, brow(s0)), arow(s0), -c0 * gau, fma(-c0, deu, ph[s0]), xa, xc, xd);
+        c2_pivot3<FP64>(fma(-c0, alu, brow(s0)), arow(s0), -c0 * gau, fma(-c0, deu, ph[s0]), xa, xc, xd);
         r8[0] = xa;
         r8[1 * C2_ROWS] = xc;
         r8[2 * C2_ROWS] = xd;
     }
-    bar_group(C2_BAR, C2_THREADS);
+    c2_bar<FP64>();
     if (live) {
         const double Ap = r8[0], Cp = r8[C2_ROWS], Dp = r8[2 * C2_ROWS];
         const double alq = r8[3 * C2_ROWS], gaq = r8[4 * C2_ROWS], deq = r8[5 * C2_ROWS];
@@ -229,7 +270,7 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
         r8[5 * C2_ROWS] = -gaq * Cn;
         r8[6 * C2_ROWS] = fma(-gaq, Dn, fma(-alq, Dp, deq));
     }
-    bar_group(C2_BAR, C2_THREADS);
+    c2_bar<FP64>();
     if (live && q == 0) {
         double gm[C2_YSEG], z[C2_YSEG];
         double gq = 0, u = 0;
@@ -239,7 +280,7 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
             const double ra = rr[3 * C2_ROWS], rb = rr[4 * C2_ROWS];
             const double rc = rr[5 * C2_ROWS], rd = rr[6 * C2_ROWS];
             const double bet = (k == 0) ? rb : fma(-ra, gq, rb);
-            pivot(bet, (k == 0) ? rd : fma(-ra, u, rd), rc, u, gq);
+            c2_pivot<FP64>(bet, (k == 0) ? rd : fma(-ra, u, rd), rc, u, gq);
             gm[k] = gq;
             z[k] = u;
         }
@@ -250,7 +291,7 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
         for (int k = 0; k < C2_YSEG; k++)
             yr[((size_t)k * C2_YSLOT + 7) * C2_ROWS + p] = z[k];
     }
-    bar_group(C2_BAR, C2_THREADS);
+    c2_bar<FP64>();
     if (live) {
         const double xl = r8[7 * C2_ROWS];
         const double zp = q ? r8[7 * C2_ROWS - C2_YSLOT * C2_ROWS] : 0.0;
@@ -260,7 +301,7 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
         for (int c = s0 + 1; c < s0 + ml - 1; c++)
             ph[c] = fma(-ga[c * C2_ROWS + p], xl, fma(-al[c * C2_ROWS + p], xf, ph[c]));
     }
-    bar_group(C2_BAR, C2_THREADS);
+    c2_bar<FP64>();
 }
 
 } // namespace dgb

@@ -207,10 +207,10 @@ __global__ void __launch_bounds__(C2_THREADS + C2_PREP) k_integrate2d_cluster(C2
             }
             bar_group(C2_BAR, C2_THREADS);
             if (!(frozen & 1))
-                c2_sweep_x(cluster, S, rank, blk, pitch, L, R0, m, al, ga, xr, zin,
+                c2_sweep_x<false>(cluster, S, rank, blk, pitch, L, R0, m, al, ga, xr, zin,
                            vecs(step, 0), ax[0], g, j0, j1);
             if (!(frozen & 2))
-                c2_sweep_y(blk, pitch, L, R0, m, al, ga, yr, vecs(step, 1), ax[1], g, j0, j1);
+                c2_sweep_y<false>(blk, pitch, L, R0, m, al, ga, yr, vecs(step, 1), ax[1], g, j0, j1);
         }
         __syncthreads();
     }

@@ -56,12 +56,13 @@ __device__ __forceinline__ double rcp_seed(double x)
 // Reciprocal to ~1 ulp: seed refined by one cubic Newton-Raphson step.  Not
 // inlined: it is the rare other side of rcp_full and pivot below, and a
 // predicated-off FP64 instruction takes the pipe like one that runs.
-static __device__ __noinline__ double rcp_newton(double x)
+__device__ __forceinline__ double rcp_newton_here(double x)
 {
     double r = rcp_seed(x);
     double e = fma(-x, r, 1.0);
     return fma(r, fma(e, e, e), r);
 }
+static __device__ __noinline__ double rcp_newton(double x) { return rcp_newton_here(x); }
 
 // The same reciprocal, and products with it, on the integer pipes.
 //
