@@ -49,17 +49,18 @@ NS = (40, 40)
 NINST = 4096
 BYTES_PER_PS = 16      # algorithmic HBM bytes per point-sweep (phi read + write)
 FLOPS_PER_PS = 30      # algorithmic FP64 flops per point-sweep (reference formulation)
-# FP64 thread instructions per point-sweep in k_integrate2d, from ncu
+# FP64 thread instructions per point-sweep in k_integrate2d_ws, from ncu
 # counters (sm__sass_thread_inst_executed_op_fp64_pred_on.sum over the
-# point-sweeps of 1024 seed-0 instances, all three grids): 10.40 (the
-# recurrence's 10 per point plus the per-step vector builds)
-FP64_INSTR_PER_PS = 10.4
+# point-sweeps of 1024 seed-0 instances, all three grids): 6.16 (five of the
+# recurrence's ten operations per point, the reciprocal and the products with
+# it being on the integer pipes, a sixth where the sub-diagonal is formed
+# twice, and the per-step vector builds)
+FP64_INSTR_PER_PS = 6.16
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of the integration of one
-# full step of this workload, by launch mode: one mixed launch, or the three
-# launches of per_grid (L = 100 and L = 80 with two items per CTA: 1.061 +
-# 0.319 GB and 0.997 + 0.176 GB; L = 90 one item per CTA: 1.033 + 0.245 GB)
-K2_TRAFFIC_BYTES = {"persistent": 2.89e9 + 0.886e9,
-                    "per_grid": (1.0611 + 1.0325 + 0.9971) * 1e9 + (318.70 + 244.73 + 175.57) * 1e6}
+# full step of this workload, the three launches of per_grid (L = 100, 90, 80;
+# nearly all of it the factors' slices written back from L2)
+K2_TRAFFIC_BYTES = {"per_grid": (1412.17 + 39.73 + 68.08) * 1e9 +
+                                (3308.94 + 2049.50 + 2822.01) * 1e9}
 
 
 def im_draws(n, seed):
@@ -514,12 +515,12 @@ def run_ours(a, world, rank, local):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic,
                      "peak_source": src,
-                     "kernel": "k_integrate2d",
+                     "kernel": "k_integrate2d_ws",
                      "launches_per_step": eng.launches_per_integrate() - 2,
                      "per": "step: achieved and traffic cover every integration launch of "
                             "one step (one per grid size with per_grid)",
                      "note": "FP64-pipe bound: phi stays in shared memory, so HBM carries "
-                             "little; see fp64"},
+                             "the write-back of the factors' slices; see fp64"},
         "fp64": {"algorithmic_tflops": fp64_achieved,
                  "pipe_tflops": fp64_instr, "peak_tflops": fp64_peak,
                  "frac": fp64_instr / fp64_peak,
