@@ -163,7 +163,7 @@ __device__ __forceinline__ void adn_tile(const ADNArgs &A, long tile_idx, double
     }
     const long l0 = tile_idx * nt;
     const int n = (int)min((long)nt, N.nlines - l0);
-    nd_tile_io(N, tile, nt, l0, n, false);
+    nd_tile_io<SG>(N, tile, nt, l0, n, false);
     __syncthreads();
     const int j0 = (g.x[0] == 0.0) ? 0 : -1;
     const int j1 = (g.x[L - 1] == 1.0) ? L - 1 : -1;
@@ -278,7 +278,7 @@ __device__ __forceinline__ void adn_tile(const ADNArgs &A, long tile_idx, double
                 G[q] = (SG > 1 || r0 == 0) ? Q[q] : G[q] + Q[q];
         }
     }
-    nd_tile_io(N, tile, nt, l0, n, true);
+    nd_tile_io<SG>(N, tile, nt, l0, n, true);
     // fixed-order sums of G: the runs of each line (in the tile's place), then
     // the 32 lines of a warp
     if (SG > 1) {

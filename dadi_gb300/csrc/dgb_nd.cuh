@@ -213,7 +213,11 @@ __device__ __forceinline__ void nd_carve(double *smem, int L, int nt, bool delj,
 
 // Load (dir=0) or store (dir=1) the CTA's tile of lines [l0, l0+n).  (Moving
 // each thread's elements in batches of 8 loads in flight measured no faster
-// on 3-D grids of L = 70-90: the sweep's time is its solve.)
+// on 3-D grids of L = 70-90: the sweep's time is its solve.)  NQ threads per
+// line, alternate points each; a constant, so that the loop over a line's
+// points is unrolled (60 constant-coefficient steps at 100^2 points 9.42 ms
+// with the count taken from blockDim, 9.17 so).
+template <int NQ = 1>
 __device__ __forceinline__ void nd_tile_io(const NDArgs &A, double *tile, int nt, long l0, int n,
                                            bool store)
 {
@@ -234,14 +238,13 @@ __device__ __forceinline__ void nd_tile_io(const NDArgs &A, double *tile, int nt
             }
         }
     } else {
-        // one thread per line, or blockDim.x / nt of them (alternate points)
-        const int q = (int)threadIdx.x / nt, nq = (int)blockDim.x / nt;
+        const int q = (NQ > 1) ? (int)threadIdx.x / nt : 0;
         const int t = (int)threadIdx.x - q * nt;
         if (t < n) {
             long line = l0 + t;
             long outer = line / A.S, inner = line - outer * A.S;
             double *g0 = A.phi + outer * A.LS + inner;
-            for (int p = q; p < L; p += nq) {
+            for (int p = q; p < L; p += NQ) {
                 if (store)
                     g0[p * A.S] = tile[p * tp + t];
                 else
