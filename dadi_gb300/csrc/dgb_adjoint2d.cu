@@ -713,6 +713,20 @@ __host__ __device__ inline size_t adw_smem_doubles(int L)
     return 2 * (size_t)L * pitch + (6 + 10 + 8 + 8 * 2 + 8 * 2) * (size_t)L;
 }
 
+// Whether k_adjoint2d has room for the adjoint of L points in shared memory.
+static bool ad_lam_fits(int L)
+{
+    return ((size_t)AD_VEC_DOUBLES * L + (size_t)L * odd_pitch(L)) * sizeof(double) +
+               sizeof(ADShared) + 4096 <= cta_smem_bytes();
+}
+
+// Whether k_adjoint2d_ws takes grids of up to L points.
+static bool adw_fits(int L)
+{
+    return (L + 31) / 32 <= ADW_MAXWARPS &&
+           adw_smem_doubles(L) * sizeof(double) + sizeof(ADWShared) + 1024 <= cta_smem_bytes();
+}
+
 // Points of a line and of the stored densities along it, with the rows of the
 // next ADW_B points loaded ahead: f(i, mu_i, p_i, r_i, mu_{i+1}, p_{i+1}).
 constexpr int ADW_B = 4;
@@ -1610,17 +1624,9 @@ static int adjoint2d_run(const int *masks, int ninst, const int *Ls, int ngrids,
         nblocks = std::min<long>(nblocks, max_blocks);
     A.scratch = (double *)((char *)ws + 256);
     size_t smem = (size_t)AD_VEC_DOUBLES * Lmax * sizeof(double);
-    {
-        // the adjoint in shared memory when vectors + Lmax x odd pitch fit
-        int dev = 0, optin = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        const int lpitch = (Lmax % 2) ? Lmax : Lmax + 1;
-        size_t with_lam = smem + (size_t)Lmax * lpitch * sizeof(double);
-        if (with_lam + sizeof(ADShared) + 4096 <= (size_t)optin) {
-            A.lam_smem = 1;
-            smem = with_lam;
-        }
+    if (ad_lam_fits(Lmax)) {
+        A.lam_smem = 1;
+        smem += (size_t)Lmax * odd_pitch(Lmax) * sizeof(double);
     }
     if (traj ? raise_smem_limit(k_adjoint2d<true>) : raise_smem_limit(k_adjoint2d<false>))
         return DGB_ERR_CUDA;
@@ -1676,17 +1682,15 @@ static int adjoint2d_run(const int *masks, int ninst, const int *Ls, int ngrids,
         // adjoint's two copies fit and the workspace holds the factors of a
         // CTA per SM (or per item)
         const int warps = (Lmax + 31) / 32;
-        int dev = 0, optin = 0, nsm = 0;
+        int dev = 0, nsm = 0;
         cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         const size_t wsmem = adw_smem_doubles(Lmax) * sizeof(double);
         const size_t slice = k2w_slice_doubles(Lmax, true) * sizeof(double);
         long want = std::min<long>(nsm, nwalk);
         if (max_blocks > 0)
             want = std::min<long>(want, max_blocks);
-        if (warps <= ADW_MAXWARPS && wsmem + sizeof(ADWShared) + 1024 <= (size_t)optin &&
-            (long)((ws_bytes - 256) / slice) >= want) {
+        if (adw_fits(Lmax) && (long)((ws_bytes - 256) / slice) >= want) {
             void (*const kernels[])(ADArgs) = {k_adjoint2d_ws<1>, k_adjoint2d_ws<2>,
                                                k_adjoint2d_ws<3>, k_adjoint2d_ws<4>};
             if (raise_smem_limit(kernels[warps - 1]))
@@ -1717,9 +1721,18 @@ extern "C" int dgb_adjoint2d(const int *masks, int ninst, const int *Ls, int ngr
 
 extern "C" size_t dgb_adjoint2d_traj_ws_bytes(int Lmax, int nblocks)
 {
-    // Thomas scratch per CTA, or half the factors of k_adjoint2d_ws's (which
-    // runs one CTA per SM where this allows two)
-    return 256 + (size_t)nblocks * dgb::k2w_slice_doubles(Lmax, true) / 2 * sizeof(double);
+    // Per CTA asked for, half the factors of one of k_adjoint2d_ws (which runs
+    // one CTA per SM where this allows two), or beyond its grids the Thomas
+    // scratch of one of k_adjoint2d; of one and a half where the adjoint is in
+    // global memory (from 153 points on) and an SM holds up to five.  Gradients
+    // of 400 sets of 20 steps at 160 points with 1-5 CTAs per SM: 97, 78, 65,
+    // 64, 69 ms; of 400 IM sets, whose longest walks set the time, 395, 399,
+    // 406, 399, 410.
+    const size_t scratch = (size_t)Lmax * Lmax, n = (size_t)nblocks;
+    const size_t doubles = dgb::adw_fits(Lmax)      ? n * dgb::k2w_slice_doubles(Lmax, true) / 2
+                           : dgb::ad_lam_fits(Lmax) ? n * scratch
+                                                    : (3 * n + 1) / 2 * scratch;
+    return 256 + doubles * sizeof(double);
 }
 
 extern "C" int dgb_adjoint2d_traj(const int *masks, int ninst, const int *Ls, int ngrids,

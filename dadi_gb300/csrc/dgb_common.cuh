@@ -438,6 +438,9 @@ __device__ __forceinline__ void axis_scalars_2d(AxisScalars &s, int a, const dou
               s.bcs, s.bce);
 }
 
+// Pitch of a density of L x L points in shared memory.
+__host__ __device__ inline int odd_pitch(int L) { return (L % 2) ? L : L + 1; }
+
 // Barrier of n threads of a CTA.
 __device__ __forceinline__ void bar_group(int id, int n)
 {

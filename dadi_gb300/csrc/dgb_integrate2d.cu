@@ -71,8 +71,6 @@ struct K2Args {
     const dgb_item2d *items; // optional explicit work items (grid, slot, schedule each)
 };
 
-__host__ __device__ inline int odd_pitch(int L) { return (L % 2) ? L : L + 1; }
-
 struct K2Layout {
     int pitch;
     size_t total;
@@ -1078,6 +1076,14 @@ static int k2w_per_sm(long nwork, int sms)
     return (int)std::max<long>(1, std::min<long>(5, nwork / (3L * sms)));
 }
 
+// Whether the split kernels take grids of up to L points: five warps of lines,
+// and the density in shared memory (159 points).
+static bool k2w_fits(int L, bool delj)
+{
+    const size_t smem = (delj ? k2d_smem_doubles(L) : k2w_smem_doubles(L)) * sizeof(double);
+    return (L + 31) / 32 <= K2W_MAXWARPS && smem + sizeof(K2WShared) + 1024 <= cta_smem_bytes();
+}
+
 // Launch k_integrate2d_ws over A's work (queue counter already cleared, or
 // null: one item per CTA) on `sms` SMs with slices from `slices` on; -1 where
 // it does not apply: grids beyond five warps of lines or shared memory, or too
@@ -1088,19 +1094,15 @@ static int k2w_per_sm(long nwork, int sms)
 // and 51.
 static int k2w_launch(K2Args &A, void *slices, size_t bytes, int sms, cudaStream_t st)
 {
-    const int warps = (A.Lmax + 31) / 32;
-    if (warps > K2W_MAXWARPS)
+    if (!k2w_fits(A.Lmax, A.use_delj))
         return -1;
+    const int warps = (A.Lmax + 31) / 32;
     const int threads = 32 * warps * (A.use_delj ? 1 + k2d_groups(warps) : k2w_groups(warps));
     const size_t smem = (A.use_delj ? k2d_smem_doubles(A.Lmax) : k2w_smem_doubles(A.Lmax)) *
                         sizeof(double);
-    int dev = 0, optin = 0, occ = 0, l2 = 0;
+    int dev = 0, occ = 0, l2 = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
-            cudaSuccess ||
         cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
-        return -1;
-    if (smem + sizeof(K2WShared) + 1024 > (size_t)optin)
         return -1;
     void (*(*const kernels[])(bool))(K2Args) = {k2w_kernel<1>, k2w_kernel<2>, k2w_kernel<3>,
                                                 k2w_kernel<4>, k2w_kernel<5>};
@@ -1169,7 +1171,17 @@ int k2_integrate_table(double *phi, int L, const double *xx, const double *table
     return k2_launch(A, 1, bytes, st);
 }
 
-size_t k2_table_ws_bytes(int L) { return k2d_slice_doubles(L) * sizeof(double); }
+// Doubles of a split kernel's slice for grids of up to L points, 0 where none
+// runs: what a workspace has to hold beyond k_integrate2d's Thomas scratch.
+static size_t k2w_slice(int L, bool delj)
+{
+    return !k2w_fits(L, delj) ? 0 : delj ? k2d_slice_doubles(L) : k2w_slice_doubles(L, true);
+}
+
+size_t k2_table_ws_bytes(int L)
+{
+    return std::max({(size_t)L * L, k2w_slice(L, false), k2w_slice(L, true)}) * sizeof(double);
+}
 
 size_t k2_batch_ws_bytes(int Lmax, long nwork)
 {
@@ -1179,8 +1191,8 @@ size_t k2_batch_ws_bytes(int Lmax, long nwork)
     auto slices = [&](int ctas, size_t slice) {
         return slice * (size_t)std::min<long>((long)sms * ctas, std::max<long>(nwork, 1));
     };
-    return 256 + sizeof(double) * std::max({scratch, slices(per_sm, k2w_slice_doubles(Lmax, true)),
-                                            slices(1, k2d_slice_doubles(Lmax))});
+    return 256 + sizeof(double) * std::max({scratch, slices(per_sm, k2w_slice(Lmax, false)),
+                                            slices(1, k2w_slice(Lmax, true))});
 }
 
 // norder: integrate only the work items order[0 .. norder) (<= 0: all);

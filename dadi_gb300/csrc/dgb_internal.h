@@ -57,6 +57,20 @@ template <typename Kernel> inline int raise_smem_limit(Kernel kernel)
     return raise_smem_limit_ptr((const void *)kernel);
 }
 
+// Shared memory a CTA can have, static and dynamic together: the current
+// device's, or sm_103a's 227 KB where there is none to ask (size queries on a
+// host without a GPU).
+inline size_t cta_smem_bytes()
+{
+    int dev = 0, optin = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) ==
+            cudaSuccess)
+        return (size_t)optin;
+    cudaGetLastError();
+    return 227 << 10;
+}
+
 // Load a kernel now (1 if it cannot be).  Under lazy module loading a
 // kernel is loaded at its first launch, and loading can wait for the device
 // to go idle: a first launch on one stream then serialises behind the work

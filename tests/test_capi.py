@@ -126,3 +126,26 @@ def test_count_steps_matches_python_schedule(lib):
             t = t + min(dt, T - t)
             k += 1
         assert abs(k - n) <= 1
+
+
+@pytest.mark.parametrize("L", [161, 200, 500, 4000])
+def test_workspace_beyond_the_split_kernels_is_scratch_only(lib, L):
+    """Grids that no split kernel takes ask for Thomas scratch alone: L x L
+    doubles per CTA, whatever the number of work items (a batch), or of one
+    integration."""
+    scratch = 8 * L * L
+    sms, rest = divmod(lib.dgb_workspace_bytes(1, 2, L, 1) - 256, 4 * scratch)
+    assert rest == 0 and sms >= 1
+    for n in (100, 3000, 100000):
+        assert lib.dgb_workspace_bytes(1, 2, L, n) == 256 + 4 * scratch * sms
+    # (one integration: or the coefficient records of the sweeps)
+    assert lib.dgb_workspace_bytes(0, 2, L, 0) <= max(scratch, 8 << 20) + (8 << 10) * L
+
+
+@pytest.mark.parametrize("L,per_cta", [(110, 1), (128, 1), (152, 1), (153, 1.5), (500, 1.5)])
+def test_trajectory_walk_workspace_beyond_the_split_walk(lib, L, per_cta):
+    """The backward walk's Thomas scratch: a CTA's for each CTA asked for, one
+    and a half where the adjoint is in global memory."""
+    for n in (1, 2, 304):
+        want = -(-int(2 * per_cta * n) // 2) * 8 * L * L
+        assert lib.dgb_adjoint2d_traj_ws_bytes(L, n) == 256 + want
