@@ -693,7 +693,7 @@ __global__ void __launch_bounds__(AD_THREADS) k_adjoint2d(ADArgs A)
 // n - 1, then of n - 2, ...).  Each sum runs over a line's points in
 // k_adjoint2d's order and each line's lane adds up its steps in that order, so
 // the gradients are bitwise the same.  Grids whose two copies fit shared memory
-// (up to 106 points).
+// (up to 105 points).
 constexpr int ADW_MAXWARPS = 4;
 constexpr int ADW_GROUPS = 6;
 
@@ -720,11 +720,12 @@ static bool ad_lam_fits(int L)
                sizeof(ADShared) + 4096 <= cta_smem_bytes();
 }
 
-// Whether k_adjoint2d_ws takes grids of up to L points.
+// Whether k_adjoint2d_ws takes grids of up to L points (105: 232,088 bytes of
+// the 232,448 that a CTA can have; the compiler rounds the static part up).
 static bool adw_fits(int L)
 {
     return (L + 31) / 32 <= ADW_MAXWARPS &&
-           adw_smem_doubles(L) * sizeof(double) + sizeof(ADWShared) + 1024 <= cta_smem_bytes();
+           adw_smem_doubles(L) * sizeof(double) + sizeof(ADWShared) + 64 <= cta_smem_bytes();
 }
 
 // Points of a line and of the stored densities along it, with the rows of the

@@ -142,10 +142,16 @@ def test_workspace_beyond_the_split_kernels_is_scratch_only(lib, L):
     assert lib.dgb_workspace_bytes(0, 2, L, 0) <= max(scratch, 8 << 20) + (8 << 10) * L
 
 
-@pytest.mark.parametrize("L,per_cta", [(110, 1), (128, 1), (152, 1), (153, 1.5), (500, 1.5)])
+@pytest.mark.parametrize("L,per_cta", [(106, 1), (110, 1), (128, 1), (152, 1), (153, 1.5), (500, 1.5)])
 def test_trajectory_walk_workspace_beyond_the_split_walk(lib, L, per_cta):
     """The backward walk's Thomas scratch: a CTA's for each CTA asked for, one
     and a half where the adjoint is in global memory."""
     for n in (1, 2, 304):
         want = -(-int(2 * per_cta * n) // 2) * 8 * L * L
         assert lib.dgb_adjoint2d_traj_ws_bytes(L, n) == 256 + want
+
+
+def test_trajectory_walk_workspace_at_the_end_of_the_split_walk(lib):
+    """Up to 105 points, whose two copies of the adjoint fit shared memory."""
+    for L in (3, 96, 104, 105):
+        assert lib.dgb_adjoint2d_traj_ws_bytes(L, 2) == 256 + 8 * 6 * L * (-(-L // 16) * 16)

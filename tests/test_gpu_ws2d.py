@@ -104,3 +104,30 @@ def test_adjoint_walk_on_groups_of_warps(cuda_lib, L, selection):
            for t in (True, False)]
     assert np.isfinite(got[1]).all() and np.abs(got[1]).max() > 0
     assert np.array_equal(got[0], got[1])
+
+
+def _gradient(L, steps, selection, trajectory):
+    import torch
+    from dadi_gb300 import batch
+    eng = batch.Batch2D((L,), (4, 4))
+    eng.cluster_adjoint, eng.cluster_forward = 0, False
+    p = _sets(5, steps, L)
+    rec, seeds = batch.im_instances(p), batch.im_seeds(5)
+    rec["frozen"][3], rec["nomut"][2] = 2, 1
+    if selection:
+        seeds["dform"][1:, 4, 0, 0] = 1.0
+    data = torch.ones(5, 5, dtype=torch.float64, device="cuda")
+    return eng.loglik_and_grad(p, data, scale=10.0, rec=rec, seeds=seeds,
+                               trajectory=trajectory)[1].cpu().numpy()
+
+
+@pytest.mark.parametrize("L", [103, 104, 105, 106])
+def test_adjoint_walk_at_the_end_of_its_range(cuda_lib, L):
+    """The last grids that k_adjoint2d_ws takes and the first that it does not
+    (the workspace query tells them apart) against the segment-mode walk."""
+    split = cuda_lib.dgb_adjoint2d_traj_ws_bytes(L, 2) > 256 + 2 * 8 * L * L
+    assert split == (L <= 105)
+    for selection in (False, True):
+        got, want = [_gradient(L, 20, selection, t) for t in (True, False)]
+        assert np.isfinite(want).all() and np.abs(want).max() > 0
+        assert np.array_equal(got, want)
