@@ -1084,56 +1084,71 @@ static bool k2w_fits(int L, bool delj)
     return (L + 31) / 32 <= K2W_MAXWARPS && smem + sizeof(K2WShared) + 1024 <= cta_smem_bytes();
 }
 
-// Launch k_integrate2d_ws over A's work (queue counter already cleared, or
-// null: one item per CTA) on `sms` SMs with slices from `slices` on; -1 where
-// it does not apply: grids beyond five warps of lines or shared memory, or too
-// little workspace.  The solves take a from the
-// workspace where the slices of all CTAs stay within the L2 cache, and form it
-// again (one more FP64 instruction a point, a third less traffic) where not:
-// 152 grids of 128 points 90 us a step with a, 62 without; of 100 points 46
-// and 51.
-static int k2w_launch(K2Args &A, void *slices, size_t bytes, int sms, cudaStream_t st)
+// The launch of a split kernel.
+struct K2WPlan {
+    void (*kernel)(K2Args);
+    int threads, keep_a;
+    size_t smem;
+    long nblocks;
+};
+
+// Plan a split kernel over nwork items on `sms` SMs with `bytes` of workspace
+// for the slices; false where none applies: grids beyond five warps of lines
+// or shared memory, or too little workspace.  The solves take a from the
+// workspace where this launch's slices are within 0.8 of the L2 cache, and
+// form it again (one more FP64 instruction a point, a third less traffic)
+// where not, whether or not the smaller slices are then within it: 152 grids
+// of 128 points 90 us a step with a, 62 without; of 100 points 46 and 51.
+static bool k2w_plan(int Lmax, bool delj_rows, long nwork, size_t bytes, int sms, K2WPlan &p)
 {
-    if (!k2w_fits(A.Lmax, A.use_delj))
-        return -1;
-    const int warps = (A.Lmax + 31) / 32;
-    const int threads = 32 * warps * (A.use_delj ? 1 + k2d_groups(warps) : k2w_groups(warps));
-    const size_t smem = (A.use_delj ? k2d_smem_doubles(A.Lmax) : k2w_smem_doubles(A.Lmax)) *
-                        sizeof(double);
+    if (!k2w_fits(Lmax, delj_rows))
+        return false;
+    const int warps = (Lmax + 31) / 32;
+    p.threads = 32 * warps * (delj_rows ? 1 + k2d_groups(warps) : k2w_groups(warps));
+    p.smem = (delj_rows ? k2d_smem_doubles(Lmax) : k2w_smem_doubles(Lmax)) * sizeof(double);
     int dev = 0, occ = 0, l2 = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
-        return -1;
+        return false;
     void (*(*const kernels[])(bool))(K2Args) = {k2w_kernel<1>, k2w_kernel<2>, k2w_kernel<3>,
                                                 k2w_kernel<4>, k2w_kernel<5>};
     void (*const delj[])(K2Args) = {k_integrate2d_delj<1>, k_integrate2d_delj<2>,
                                     k_integrate2d_delj<3>, k_integrate2d_delj<4>,
                                     k_integrate2d_delj<5>};
-    void (*kernel)(K2Args) = nullptr;
-    long nblocks = 0;
-    for (int keep = 1; keep >= (A.use_delj || k2w_groups(warps) == 3 ? 1 : 0); keep--) {
+    const int last = (delj_rows || k2w_groups(warps) == 3) ? 1 : 0;
+    for (p.keep_a = 1;; p.keep_a--) {
         const size_t slice =
-            (A.use_delj ? k2d_slice_doubles(A.Lmax) : k2w_slice_doubles(A.Lmax, keep)) *
+            (delj_rows ? k2d_slice_doubles(Lmax) : k2w_slice_doubles(Lmax, p.keep_a)) *
             sizeof(double);
-        kernel = A.use_delj ? delj[warps - 1] : kernels[warps - 1](keep);
-        if (raise_smem_limit(kernel))
-            return -1;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) !=
+        p.kernel = delj_rows ? delj[warps - 1] : kernels[warps - 1](p.keep_a);
+        if (raise_smem_limit(p.kernel))
+            return false;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p.kernel, p.threads, p.smem) !=
             cudaSuccess) {
             cudaGetLastError();
-            return -1;
+            return false;
         }
-        const long want = std::min<long>((long)sms * std::min(occ, k2w_per_sm(A.nwork, sms)),
-                                         A.nwork);
-        nblocks = std::min<long>((long)(bytes / slice), want);
-        if (nblocks == want && (size_t)nblocks * slice <= (size_t)l2 / 10 * 8)
+        const long want = std::min<long>((long)sms * std::min(occ, k2w_per_sm(nwork, sms)),
+                                         nwork);
+        p.nblocks = std::min<long>((long)(bytes / slice), want);
+        if (p.keep_a == last ||
+            (p.nblocks == want && (size_t)p.nblocks * slice <= (size_t)l2 / 10 * 8))
             break;
     }
-    if (nblocks < std::min(sms, A.nwork))
+    return p.nblocks >= std::min<long>(sms, nwork);
+}
+
+// Launch a split kernel over A's work (queue counter already cleared, or null:
+// one item per CTA) on `sms` SMs with slices from `slices` on; -1 where none
+// applies.
+static int k2w_launch(K2Args &A, void *slices, size_t bytes, int sms, cudaStream_t st)
+{
+    K2WPlan p;
+    if (!k2w_plan(A.Lmax, A.use_delj, A.nwork, bytes, sms, p))
         return -1;
     A.gam_smem = 0;
     A.gam_glob = (double *)slices;
-    kernel<<<(unsigned)nblocks, threads, smem, st>>>(A);
+    p.kernel<<<(unsigned)p.nblocks, p.threads, p.smem, st>>>(A);
     return cudaGetLastError() == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
 }
 
@@ -1537,6 +1552,21 @@ extern "C" int dgb_items2d_integrate(const dgb_item2d *items, int nitems, int Lm
     if (cudaMemsetAsync(A.counter, 0, sizeof(int), (cudaStream_t)stream) != cudaSuccess)
         return DGB_ERR_CUDA;
     return k2_launch(A, nblocks, smem, (cudaStream_t)stream, threads);
+}
+
+extern "C" int dgb_probe_split2d(int Lmax, long nwork, int use_delj_trick, size_t ws_bytes,
+                                 int *ctas, int *keep_a)
+{
+    using namespace dgb;
+    if (Lmax < 3 || nwork < 1 || !ctas || !keep_a)
+        return DGB_ERR_ARG;
+    K2WPlan p;
+    if (ws_bytes < 256 ||
+        !k2w_plan(Lmax, use_delj_trick != 0, nwork, ws_bytes - 256, k2_num_sms(), p))
+        return DGB_ERR_UNSUPPORTED;
+    *ctas = (int)p.nblocks;
+    *keep_a = p.keep_a;
+    return DGB_OK;
 }
 
 extern "C" int dgb_sched2d_host(const dgb_inst2d *insts, int ninst,

@@ -613,11 +613,19 @@ int dgb_integrate2d_noalloc(double *phi, int L, const double *xx, const double *
  * dgb_probe_pivot: for xtc = x[n], t[n], c[n] (device), out = t * (1/x),
  * c * (1/x), t / x and c * x as the sweeps' integer arithmetic gives them,
  * then the same four as FP64 instructions give them (8 n doubles), so tests
- * can compare the bits. */
+ * can compare the bits.
+ * dgb_probe_split2d: the launch that the automatic shape of
+ * dgb_batch2d_integrate and dgb_items2d_integrate (not one_per_cta) takes for
+ * nwork items on grids of up to Lmax points with ws_bytes of workspace: its
+ * CTAs and whether its solves read the rows' subdiagonals from the workspace
+ * (*keep_a 1) or form them again (0); DGB_ERR_UNSUPPORTED where one warp runs
+ * factors and solves of its lines. */
 int dgb_probe_fp64_fma(double *out, int blocks, int threads, int iters, int active_lanes,
                        void *stream);
 int dgb_probe_rcp(const double *x, double *out, int n, void *stream);
 int dgb_probe_pivot(const double *xtc, double *out, int n, void *stream);
+int dgb_probe_split2d(int Lmax, long nwork, int use_delj_trick, size_t ws_bytes, int *ctas,
+                      int *keep_a);
 
 #ifdef __cplusplus
 }

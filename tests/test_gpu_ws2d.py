@@ -106,6 +106,40 @@ def test_adjoint_walk_on_groups_of_warps(cuda_lib, L, selection):
     assert np.array_equal(got[0], got[1])
 
 
+def _form(lib, L, n, delj=False):
+    """(CTAs per SM, whether a is kept) of the split kernels' launch over n
+    grids of L points, or None where k_integrate2d serves."""
+    import ctypes
+    import torch
+    from dadi_gb300 import _lib
+    ctas, keep = ctypes.c_int(), ctypes.c_int()
+    rc = lib.dgb_probe_split2d(L, n, int(delj), lib.dgb_workspace_bytes(1, 2, L, n),
+                               ctypes.byref(ctas), ctypes.byref(keep))
+    if rc != 0:
+        assert rc == _lib.DGB_ERR_UNSUPPORTED
+        return None
+    return ctas.value / torch.cuda.get_device_properties(0).multi_processor_count, keep.value
+
+
+@pytest.mark.parametrize("L,n,keep", [(31, 2400, 1), (64, 1500, 1), (80, 920, 1), (90, 920, 0),
+                                      (100, 920, 0), (128, 170, 0), (130, 170, 0)])
+def test_same_bits_with_full_sms(cuda_lib, L, n, keep):
+    """Several CTAs per SM (as many as shared memory and registers hold), and
+    both forms of the solve at three to five warps of lines."""
+    from dadi_gb300 import batch
+    per_sm, kept = _form(cuda_lib, L, n)
+    assert kept == keep
+    assert per_sm >= (3 if L <= 64 else 2 if L <= 100 else 1)
+    got, want = _both(L, batch.im_instances(_sets(n, 4, 3)))
+    assert np.array_equal(got, want)
+
+
+def test_end_of_the_split_kernels_range(cuda_lib):
+    """159 points are the last that the split kernels take."""
+    for delj in (False, True):
+        assert _form(cuda_lib, 159, 3, delj) and _form(cuda_lib, 160, 3, delj) is None
+
+
 def _gradient(L, steps, selection, trajectory):
     import torch
     from dadi_gb300 import batch
