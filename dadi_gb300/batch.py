@@ -347,7 +347,8 @@ class Batch2D:
         when schedules are per grid (use_old_timestep)."""
         torch = self.torch
         lib = _lib.lib()
-        st = settings_from_globals(self.gam_placement, self.threads)
+        # (-2: automatic, for launches that share the SMs)
+        st = settings_from_globals(self.gam_placement, self.threads or -2)
         if st.use_old_timestep:
             return None
         n = len(rec)

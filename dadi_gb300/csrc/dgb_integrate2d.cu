@@ -40,7 +40,7 @@ namespace dgb {
 constexpr int K2_THREADS = 128;
 constexpr int K2_MAXG = DGB_B2_MAXG;
 constexpr int K2_ROW = 11; // DGB_ROW_STRIDE(2)
-constexpr int K2_AUTO_ANY_L = -2; // dgb_settings.threads: as 0
+constexpr int K2_AUTO_SHARED = -2; // dgb_settings.threads: as 0, beside other launches
 
 struct K2Args {
     int ngrids;
@@ -69,6 +69,8 @@ struct K2Args {
     const long *ckpt_off;  // first checkpoint double of each work id
     int ckpt_every;
     const dgb_item2d *items; // optional explicit work items (grid, slot, schedule each)
+    int *live;               // k_integrate2d_ws, CHOSEN: CTAs per SM that run, then the
+                             // number of CTAs started on each SM
 };
 
 struct K2Layout {
@@ -334,7 +336,87 @@ __host__ __device__ inline size_t k2w_smem_doubles(int L)
 // vectors would hold up the solves) the vectors.
 __host__ __device__ constexpr int k2w_groups(int W) { return W <= 2 ? 3 : 2; }
 
-template <int W, bool KEEP_A>
+// How much one of k CTAs of W warps of lines on an SM is slower than one alone
+// (grids of 24 and 31 points, k = 2 .. 5: 1.12 1.18 1.30 1.60 and 1.05 1.07
+// 1.12 1.24; of 45 and 64, k = 2 .. 4: 1.14 1.38 1.79 and 1.22 1.60 2.14).
+__host__ __device__ constexpr float k2w_slowdown(int W, int k)
+{
+    return 1.0f + (W == 1 ? 0.1f : 0.3f) * (k - 1);
+}
+
+// k2w_live serves launches of fewer than K2W_HEADS - 1 items per SM (from there
+// on k2w_per_sm gives all the CTAs that fit).
+constexpr int K2W_HEADS = 16;
+constexpr int K2W_LIVE_THREADS = 256;
+constexpr int K2W_SMIDS = 1023; // (SMs are told apart by their number below this)
+
+// Whether a CTA, asked once at its start, is beyond those of its SM that run.
+__device__ __forceinline__ bool k2w_leaves(int *live)
+{
+    unsigned sm;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+    return atomicAdd(live + 1 + sm % K2W_SMIDS, 1) >= *live;
+}
+
+// How many CTAs per SM of a launch with a few items per SM run: `most` are
+// launched, and those beyond leave (k2w_leaves; going by SM and not by
+// blockIdx, as the first CTAs need not be on different SMs).  Such a batch ends
+// with its longest item, and further CTAs on an SM slow that one down; but
+// items of like length end sooner the more of them run at once.  With k CTAs
+// per SM it takes, in units of an item's cost alone, at least its work spread
+// evenly, and j + 1 times the cost of the item at place j k sms of the order
+// (longest first); to that comes what they slow each other down while all of
+// them have work.  The k with the least runs.  A kernel of its own, and asked
+// where a CTA takes its items: more code at the head of k_integrate2d_ws gave
+// its loop other registers and cost 4-6 %.
+// Milliseconds with k2w_per_sm's count and so: 320 sets of 100 steps at 31
+// points 4.01 and 1.63, at 64 7.16 and 3.87; 160 such at 40/50/60 points 7.44
+// and 4.05; 320 sets of 30 to 170 steps at 31/38/45 6.13 and 5.00; IM sets,
+// whose longest schedule is a dozen times the mean: 257 at 31/38/45 90 and 88,
+// 700 131 and 107, 320 at 40/50/60 126 and 108, 700 170 and 135.
+__global__ void __launch_bounds__(K2W_LIVE_THREADS)
+    k2w_live(K2Args A, int warps, int sms, int most, int *live)
+{
+    __shared__ float head[K2W_HEADS], part[K2W_LIVE_THREADS / 32];
+    const int tid = threadIdx.x;
+    for (int i = tid; i < K2W_SMIDS; i += K2W_LIVE_THREADS)
+        live[1 + i] = 0;
+    auto cost = [&](int w) {
+        const K2Item I = k2_item(A, A.order[w]);
+        return (float)(I.nsteps + 2) * (float)I.L; // (2: an item's set-up)
+    };
+    float sum = 0;
+    for (int w = tid; w < A.nwork; w += K2W_LIVE_THREADS)
+        sum += cost(w);
+    for (int off = 16; off > 0; off >>= 1)
+        sum += __shfl_down_sync(0xffffffffu, sum, off);
+    if ((tid & 31) == 0)
+        part[tid >> 5] = sum;
+    if (tid < K2W_HEADS)
+        head[tid] = ((long)tid * sms < A.nwork) ? cost(tid * sms) : 0.0f;
+    __syncthreads();
+    if (tid > 0)
+        return;
+    sum = 0;
+    for (int w = 0; w < K2W_LIVE_THREADS / 32; w++)
+        sum += part[w];
+    int best = 1;
+    float shortest = INFINITY;
+    for (int k = 1; k <= most; k++) {
+        const float even = sum / (float)(k * sms);
+        float t = even;
+        for (int j = 0; j * k < K2W_HEADS; j++)
+            t = fmaxf(t, (float)(j + 1) * head[j * k]);
+        t += (k2w_slowdown(warps, k) - 1.0f) * even;
+        if (t < shortest) {
+            best = k;
+            shortest = t;
+        }
+    }
+    *live = best;
+}
+
+template <int W, bool KEEP_A, bool CHOSEN = false>
 __global__ void __launch_bounds__(32 * W * k2w_groups(W), W == 1 ? 5 : W == 2 ? 3 : 2)
     k_integrate2d_ws(K2Args A)
 {
@@ -370,7 +452,10 @@ __global__ void __launch_bounds__(32 * W * k2w_groups(W), W == 1 ? 5 : W == 2 ? 
 
     for (int iter = 0;; iter++) {
         if (tid == 0)
-            S.item = A.counter ? atomicAdd(A.counter, 1) : (iter == 0 ? (int)blockIdx.x : A.nwork);
+            S.item = (CHOSEN && iter == 0 && k2w_leaves(A.live)) ? A.nwork
+                     : A.counter                                 ? atomicAdd(A.counter, 1)
+                     : iter == 0                                 ? (int)blockIdx.x
+                                                                 : A.nwork;
         __syncthreads();
         const int w = S.item;
         if (w >= A.nwork)
@@ -1040,7 +1125,7 @@ static int k2_num_sms()
 static int k2_pick_threads(const dgb_settings *settings, bool delj, size_t smem, int Lmax,
                            int &occ)
 {
-    const int want = (settings->threads == K2_AUTO_ANY_L) ? 0 : settings->threads;
+    const int want = (settings->threads == K2_AUTO_SHARED) ? 0 : settings->threads;
     if (want != 0 && want != 64 && want != 96 && want != 128)
         return 0;
     int warps = std::min(4, std::max(2, (Lmax + 31) / 32));
@@ -1061,7 +1146,7 @@ template <int W> static void (*k2w_kernel(bool keep_a))(K2Args)
 // Whether the caller leaves the shape of a batched launch to the rules here.
 static bool k2w_auto(const dgb_settings *s)
 {
-    return (s->threads == 0 || s->threads == K2_AUTO_ANY_L) && s->gam_placement != 1;
+    return (s->threads == 0 || s->threads == K2_AUTO_SHARED) && s->gam_placement != 1;
 }
 
 // CTAs of k_integrate2d_ws per SM for nwork items on sms SMs.  One CTA uses
@@ -1084,13 +1169,41 @@ static bool k2w_fits(int L, bool delj)
     return (L + 31) / 32 <= K2W_MAXWARPS && smem + sizeof(K2WShared) + 1024 <= cta_smem_bytes();
 }
 
+constexpr size_t K2W_LIVE_BYTES = (1 + K2W_SMIDS) * sizeof(int);
+
 // The launch of a split kernel.
 struct K2WPlan {
     void (*kernel)(K2Args);
     int threads, keep_a;
+    int most;       // CTAs per SM of which k2w_live chooses (0: all run)
+    size_t live_at; // K2W_LIVE_BYTES of the workspace for it
     size_t smem;
     long nblocks;
 };
+
+// Bytes of slices that k_integrate2d_ws keeps within L2.
+static size_t k2w_l2_budget()
+{
+    int dev = 0, l2 = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return (size_t)l2 / 10 * 8;
+}
+
+// CTAs per SM of which k2w_live chooses, of `fit` that an SM holds: at most one
+// per item, and slices within L2; or k2w_per_sm's if those are more.  0 where
+// it does not choose.
+static int k2w_most_per_sm(int Lmax, long nwork, int sms, int fit)
+{
+    if (k2w_groups((Lmax + 31) / 32) != 3 || nwork <= sms || nwork >= (long)(K2W_HEADS - 1) * sms)
+        return 0;
+    const size_t all = (size_t)sms * k2w_slice_doubles(Lmax, true) * sizeof(double);
+    const long most = std::min<long>((nwork + sms - 1) / sms, (long)(k2w_l2_budget() / all));
+    return (int)std::min<long>(fit, std::max<long>(most, k2w_per_sm(nwork, sms)));
+}
 
 // Plan a split kernel over nwork items on `sms` SMs with `bytes` of workspace
 // for the slices; false where none applies: grids beyond five warps of lines
@@ -1099,17 +1212,18 @@ struct K2WPlan {
 // form it again (one more FP64 instruction a point, a third less traffic)
 // where not, whether or not the smaller slices are then within it: 152 grids
 // of 128 points 90 us a step with a, 62 without; of 100 points 46 and 51.
-static bool k2w_plan(int Lmax, bool delj_rows, long nwork, size_t bytes, int sms, K2WPlan &p)
+// choose: k2w_live may choose the CTAs per SM.
+static bool k2w_plan(int Lmax, bool delj_rows, long nwork, size_t bytes, int sms, bool choose,
+                     K2WPlan &p)
 {
     if (!k2w_fits(Lmax, delj_rows))
         return false;
     const int warps = (Lmax + 31) / 32;
     p.threads = 32 * warps * (delj_rows ? 1 + k2d_groups(warps) : k2w_groups(warps));
     p.smem = (delj_rows ? k2d_smem_doubles(Lmax) : k2w_smem_doubles(Lmax)) * sizeof(double);
-    int dev = 0, occ = 0, l2 = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
-        return false;
+    p.most = 0;
+    int occ = 0;
+    const size_t budget = k2w_l2_budget();
     void (*(*const kernels[])(bool))(K2Args) = {k2w_kernel<1>, k2w_kernel<2>, k2w_kernel<3>,
                                                 k2w_kernel<4>, k2w_kernel<5>};
     void (*const delj[])(K2Args) = {k_integrate2d_delj<1>, k_integrate2d_delj<2>,
@@ -1132,22 +1246,45 @@ static bool k2w_plan(int Lmax, bool delj_rows, long nwork, size_t bytes, int sms
                                          nwork);
         p.nblocks = std::min<long>((long)(bytes / slice), want);
         if (p.keep_a == last ||
-            (p.nblocks == want && (size_t)p.nblocks * slice <= (size_t)l2 / 10 * 8))
+            (p.nblocks == want && (size_t)p.nblocks * slice <= budget)) {
+            const int most =
+                (delj_rows || !choose) ? 0 : k2w_most_per_sm(Lmax, nwork, sms, occ);
+            if (most > 1 && (size_t)sms * most * slice + K2W_LIVE_BYTES <= bytes) {
+                p.most = most;
+                p.kernel = warps == 1 ? k_integrate2d_ws<1, true, true>
+                                      : k_integrate2d_ws<2, true, true>;
+                if (raise_smem_limit(p.kernel))
+                    return false;
+                p.nblocks = (long)sms * most;
+                p.live_at = (size_t)p.nblocks * slice;
+            }
             break;
+        }
     }
     return p.nblocks >= std::min<long>(sms, nwork);
 }
 
 // Launch a split kernel over A's work (queue counter already cleared, or null:
 // one item per CTA) on `sms` SMs with slices from `slices` on; -1 where none
-// applies.
-static int k2w_launch(K2Args &A, void *slices, size_t bytes, int sms, cudaStream_t st)
+// applies.  alone: no other launch is meant to run beside this one (the CTAs
+// that k2w_live sends home would take places from another's, and other CTAs on
+// the SMs upset its estimate: launches per grid, 257 IM sets at 31/38/45
+// points, 95.4 ms without it and 101 with it).
+static int k2w_launch(K2Args &A, void *slices, size_t bytes, int sms, bool alone,
+                      cudaStream_t st)
 {
     K2WPlan p;
-    if (!k2w_plan(A.Lmax, A.use_delj, A.nwork, bytes, sms, p))
+    if (!k2w_plan(A.Lmax, A.use_delj, A.nwork, bytes, sms, alone && A.order, p))
         return -1;
     A.gam_smem = 0;
     A.gam_glob = (double *)slices;
+    if (p.most) {
+        int *live = (int *)((char *)slices + p.live_at);
+        k2w_live<<<1, K2W_LIVE_THREADS, 0, st>>>(A, (A.Lmax + 31) / 32, sms, p.most, live);
+        if (cudaGetLastError() != cudaSuccess)
+            return DGB_ERR_CUDA;
+        A.live = live;
+    }
     p.kernel<<<(unsigned)p.nblocks, p.threads, p.smem, st>>>(A);
     return cudaGetLastError() == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
 }
@@ -1171,7 +1308,7 @@ int k2_integrate_table(double *phi, int L, const double *xx, const double *table
     A.use_delj = use_delj;
     size_t bytes;
     if (ws) {
-        const int rc = k2w_launch(A, ws, ws_bytes, 1, st);
+        const int rc = k2w_launch(A, ws, ws_bytes, 1, true, st);
         if (rc != -1)
             return rc;
     }
@@ -1200,14 +1337,17 @@ size_t k2_table_ws_bytes(int L)
 
 size_t k2_batch_ws_bytes(int Lmax, long nwork)
 {
-    const int sms = k2_num_sms();
+    const int sms = k2_num_sms(), fit = Lmax <= 64 ? 5 : 2;
     const size_t scratch = (size_t)sms * 4 * Lmax * Lmax; // k_integrate2d, up to four CTAs per SM
-    const int per_sm = std::min(k2w_per_sm(nwork, sms), Lmax <= 64 ? 5 : 2);
-    auto slices = [&](int ctas, size_t slice) {
-        return slice * (size_t)std::min<long>((long)sms * ctas, std::max<long>(nwork, 1));
-    };
-    return 256 + sizeof(double) * std::max({scratch, slices(per_sm, k2w_slice(Lmax, false)),
-                                            slices(1, k2w_slice(Lmax, true))});
+    const size_t slice = k2w_slice(Lmax, false);
+    const long n = std::max<long>(nwork, 1);
+    size_t doubles = std::max(
+        {scratch, slice * std::min<long>((long)sms * std::min(k2w_per_sm(n, sms), fit), n),
+         k2w_slice(Lmax, true) * std::min<long>(sms, n)});
+    const int most = slice ? k2w_most_per_sm(Lmax, n, sms, fit) : 0;
+    if (most > 1)
+        doubles = std::max(doubles, slice * sms * most + K2W_LIVE_BYTES / sizeof(double));
+    return 256 + doubles * sizeof(double);
 }
 
 // norder: integrate only the work items order[0 .. norder) (<= 0: all);
@@ -1301,7 +1441,8 @@ int k2_batch(int ninst, const int *masks, const int *Ls, int ngrids, const doubl
         if (cudaMemsetAsync(A.counter, 0, sizeof(int), st) != cudaSuccess)
             return DGB_ERR_CUDA;
         const int rc = k2w_launch(A, (char *)ws + 256, ws_bytes - 256,
-                                  reserve_sms > 0 ? std::max(1, nsm - reserve_sms) : nsm, st);
+                                  reserve_sms > 0 ? std::max(1, nsm - reserve_sms) : nsm,
+                                  reserve_sms <= 0 && settings->threads != K2_AUTO_SHARED, st);
         if (rc != -1)
             return rc;
     }
@@ -1522,7 +1663,7 @@ extern "C" int dgb_items2d_integrate(const dgb_item2d *items, int nitems, int Lm
         if (cudaMemsetAsync(A.counter, 0, sizeof(int), (cudaStream_t)stream) != cudaSuccess)
             return DGB_ERR_CUDA;
         const int rc = k2w_launch(A, (char *)ws + 256, ws_bytes - 256, k2_num_sms(),
-                                  (cudaStream_t)stream);
+                                  settings->threads != K2_AUTO_SHARED, (cudaStream_t)stream);
         if (rc != -1)
             return rc;
     }
@@ -1562,7 +1703,7 @@ extern "C" int dgb_probe_split2d(int Lmax, long nwork, int use_delj_trick, size_
         return DGB_ERR_ARG;
     K2WPlan p;
     if (ws_bytes < 256 ||
-        !k2w_plan(Lmax, use_delj_trick != 0, nwork, ws_bytes - 256, k2_num_sms(), p))
+        !k2w_plan(Lmax, use_delj_trick != 0, nwork, ws_bytes - 256, k2_num_sms(), true, p))
         return DGB_ERR_UNSUPPORTED;
     *ctas = (int)p.nblocks;
     *keep_a = p.keep_a;
@@ -1592,7 +1733,8 @@ namespace dgb {
 int preload_integrate2d()
 {
     return preload(k_integrate2d<false>) + preload(k_integrate2d<true>) +
-           preload(k2w_kernel<1>(true)) +
+           preload(k2w_live) + preload(k_integrate2d_ws<1, true, true>) +
+           preload(k_integrate2d_ws<2, true, true>) + preload(k2w_kernel<1>(true)) +
            preload(k2w_kernel<2>(true)) + preload(k2w_kernel<3>(true)) +
            preload(k2w_kernel<4>(true)) + preload(k2w_kernel<5>(true)) +
            preload(k2w_kernel<1>(false)) + preload(k2w_kernel<2>(false)) +

@@ -71,9 +71,11 @@ typedef struct {
     int use_old_timestep;        /* default 0 */
     int use_delj_trick;          /* default 0 */
     int gam_placement;           /* batched engine: 0 auto, 1 shared memory, 2 workspace */
-    int threads;                 /* batched engine: 0 (or -2) auto -- a lane per line of the
-                                    largest grid for the solves and as many for the factors
-                                    of the next sweep -- or 64 / 96 / 128 threads per CTA,
+    int threads;                 /* batched engine: 0 auto -- a lane per line of the largest
+                                    grid for the solves and as many for the factors of the
+                                    next sweep -- or -2, auto for a launch beside others
+                                    (its CTAs per SM go by the number of items alone, not by
+                                    their lengths too), or 64 / 96 / 128 threads per CTA,
                                     one lane for both, where that many threads hold every
                                     line (else the fewest warps, 2-4, that do);
                                     gam_placement 1 always takes the latter.  Under the
@@ -616,8 +618,9 @@ int dgb_integrate2d_noalloc(double *phi, int L, const double *xx, const double *
  * can compare the bits.
  * dgb_probe_split2d: the launch that the automatic shape of
  * dgb_batch2d_integrate and dgb_items2d_integrate (not one_per_cta) takes for
- * nwork items on grids of up to Lmax points with ws_bytes of workspace: its
- * CTAs and whether its solves read the rows' subdiagonals from the workspace
+ * nwork ordered items on grids of up to Lmax points with ws_bytes of
+ * workspace: its CTAs (some of which may leave the items to the others) and
+ * whether its solves read the rows' subdiagonals from the workspace
  * (*keep_a 1) or form them again (0); DGB_ERR_UNSUPPORTED where one warp runs
  * factors and solves of its lines. */
 int dgb_probe_fp64_fma(double *out, int blocks, int threads, int iters, int active_lanes,

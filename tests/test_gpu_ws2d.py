@@ -134,6 +134,25 @@ def test_same_bits_with_full_sms(cuda_lib, L, n, keep):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("L,n", [(3, 160), (31, 153), (31, 700), (32, 400), (33, 400), (47, 310),
+                                 (64, 400)])
+@pytest.mark.parametrize("spread", [0.0, 1.0, 12.0])
+def test_same_bits_where_ctas_choose_to_run(cuda_lib, L, n, spread):
+    """A few items per SM: more CTAs are launched than SMs, and those beyond
+    run if the schedules are of similar length (all alike; from none to twice
+    the mean; one of 13 times the others)."""
+    from dadi_gb300 import batch
+    per_sm, kept = _form(cuda_lib, L, n)
+    assert per_sm > 1 and kept
+    p = _sets(n, 6, 4)
+    if spread == 1.0:
+        p[:, 3] *= np.linspace(0, 2, n)
+    elif spread:
+        p[n // 2, 3] *= 1 + spread
+    got, want = _both(L, batch.im_instances(p))
+    assert np.array_equal(got, want)
+
+
 def test_end_of_the_split_kernels_range(cuda_lib):
     """159 points are the last that the split kernels take."""
     for delj in (False, True):
