@@ -29,8 +29,8 @@ EXPORTS = ["dgb_abi_version", "dgb_status_string", "dgb_workspace_bytes",
            "dgb_tridiag_batch", "dgb_implicit_sweep", "dgb_implicit_precalc_sweep",
            "dgb_integrate_table", "dgb_integrate_precalc", "dgb_sched2d",
            "dgb_batch2d_integrate", "dgb_batch2d_count_steps", "dgb_probe_fp64_fma",
-           "dgb_probe_rcp", "dgb_probe_pivot", "dgb_probe_split2d",
-           "dgb_integrate2d_noalloc", "dgb_sched2d_deriv",
+           "dgb_probe_rcp", "dgb_probe_pivot", "dgb_probe_pivot3",
+           "dgb_probe_split2d", "dgb_integrate2d_noalloc", "dgb_sched2d_deriv",
            "dgb_batch2d_integrate_ckpt", "dgb_adjoint2d_scratch_bytes", "dgb_adjoint2d",
            "dgb_items2d_integrate", "dgb_sched2d_host", "dgb_from_phi2d_smem_bytes",
            "dgb_from_phi2d", "dgb_extrap_ll", "dgb_integrate_table_states",
@@ -125,6 +125,7 @@ def _declare(L):
         "dgb_probe_fp64_fma": (i, [_vp, i, i, i, i, _vp]),
         "dgb_probe_rcp": (i, [_vp, _vp, i, _vp]),
         "dgb_probe_pivot": (i, [_vp, _vp, i, _vp]),
+        "dgb_probe_pivot3": (i, [_vp, _vp, i, _vp]),
         "dgb_probe_split2d": (i, [i, lg, i, sz, ctypes.POINTER(i), ctypes.POINTER(i)]),
         "dgb_integrate2d_noalloc": (i, [_vp, i, _vp, _vp, i, i, i, i, _vp]),
         "dgb_sched2d_deriv": (i, [_vp, _vp, i, i, _vp, ctypes.POINTER(Settings), _vp, _vp, _vp,

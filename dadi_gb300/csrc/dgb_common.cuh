@@ -53,9 +53,10 @@ __device__ __forceinline__ double rcp_seed(double x)
     return r;
 }
 
-// Reciprocal to ~1 ulp: seed refined by one cubic Newton-Raphson step.  Not
-// inlined: it is the rare other side of rcp_full and pivot below, and a
-// predicated-off FP64 instruction takes the pipe like one that runs.
+// Reciprocal to ~1 ulp: seed refined by one cubic Newton-Raphson step.
+// rcp_newton is not inlined: it is the rare other side of rcp_full and pivot
+// below, and a predicated-off FP64 instruction takes the pipe like one that
+// runs.
 __device__ __forceinline__ double rcp_newton_here(double x)
 {
     double r = rcp_seed(x);
@@ -86,8 +87,6 @@ static __device__ __noinline__ double rcp_newton(double x) { return rcp_newton_h
 // = r0 2^21 (21 bits), -X rho mod 2^64 is the residual e = 1 - m r0 (|e| <
 // 2^-19) in units of 2^-73, exactly; then 1/m = r0 (1 + e + e^2) is built in
 // units of 2^-96 with an error below 2^-67, and rounded to 53 bits.
-static __device__ __noinline__ double mul_fp64(double x, double y) { return x * y; }
-
 struct Mant {
     unsigned h, l; // 2^64 / m rounded to 53 bits: the top bit of h is set
 };
@@ -192,9 +191,50 @@ __device__ __forceinline__ void rcp_wide(double x, unsigned (&r)[3])
     r[2] = (unsigned)(y >> 32);
 }
 
+static __device__ __noinline__ double mul_fp64(double x, double y) { return x * y; }
+
+// The rare sides of functions among whose operands zero is an ordinary value
+// (a model without migration or selection: every coupling to the row before the
+// first segment of a partitioned line, every mean change under the delj trick):
+// a zero's product or quotient is formed off the FP64 pipe, all else by it.
+// Not inlined, see rcp_newton.  Without migration and selection, milliseconds
+// with every zero on the FP64 pipe / so: 60 steps under the delj trick at 100
+// points 25.2 / 15.4 (with migration 17.1 / 17.0), 300 steps on clusters at 128
+// points 11.8 / 10.0, 60 steps of three populations at 90 points 5.42 / 4.99.
+// The lines' other products (pivot, mul_full) keep the plain call: they meet a
+// zero once a line, and in k_integrate2d_ws these sides cost 1-10 %.
+__device__ __forceinline__ bool is_zero(double x)
+{
+    return ((unsigned)__double2hiint(x) << 1 | (unsigned)__double2loint(x)) == 0;
+}
+
+__device__ __forceinline__ bool is_finite(double x)
+{
+    return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
+}
+
+// Zero with the sign of x * y.
+__device__ __forceinline__ double zero_of(double x, double y)
+{
+    return __hiloint2double((__double2hiint(x) ^ __double2hiint(y)) & (int)0x80000000u, 0);
+}
+
+static __device__ __noinline__ double mul_rare(double x, double y)
+{
+    if ((is_zero(x) && is_finite(y)) || (is_zero(y) && is_finite(x)))
+        return zero_of(x, y);
+    return x * y;
+}
+
+static __device__ __noinline__ double div_rare(double x, double y)
+{
+    if (is_zero(x) && !is_zero(y) && is_finite(y))
+        return zero_of(x, y);
+    return __ddiv_rn(x, y);
+}
+
 // (The delj rows have five divisions a point: 64 IM sets at pts 40/50/60 took
 // 1.33 s with them on the FP64 pipe, 0.89 with div_full.)
-static __device__ __noinline__ double div_fp64(double x, double y) { return __ddiv_rn(x, y); }
 
 // x / y rounded as IEEE division rounds, from y's rcp_wide.  A quotient is
 // never half way between two doubles, and one within the error of it (one in
@@ -222,7 +262,7 @@ __device__ __forceinline__ double div_wide(double x, double y, const unsigned (&
                                       (yh & 0xfff00000u) + (w3 & 0x100000u)),
                                 (int)(unsigned)m);
     if (bad)
-        q = div_fp64(x, y);
+        q = div_rare(x, y);
     return q;
 }
 
@@ -233,8 +273,9 @@ __device__ __forceinline__ double div_full(double x, double y)
     return div_wide(x, y, r);
 }
 
-// x * y rounded as IEEE multiplication rounds (y an unpacked double).
-__device__ __forceinline__ double mul_full(double x, double y)
+// x * y rounded as IEEE multiplication rounds (y an unpacked double); ZEROS:
+// for operands of which zero is an ordinary value.
+template <bool ZEROS = false> __device__ __forceinline__ double mul_full(double x, double y)
 {
     const unsigned yh = (unsigned)__double2hiint(y), yl = (unsigned)__double2loint(y);
     Mant m;
@@ -243,7 +284,7 @@ __device__ __forceinline__ double mul_full(double x, double y)
     bool bad = (yh & 0x7fffffffu) - 0x37f00000u >= 0x10000000u;
     double r = mul_mant(x, m, (yh & 0xfff00000u) - 0x40000000u, bad);
     if (bad)
-        r = mul_fp64(x, y);
+        r = ZEROS ? mul_rare(x, y) : mul_fp64(x, y);
     return r;
 }
 
@@ -274,19 +315,40 @@ static __device__ __noinline__ double3 pivot3_fp64(double bet, double t, double 
     return make_double3(t * inv, c * inv, d * inv);
 }
 
+// A product with 1/bet that mul_mant refused: a zero put right, or not all are.
+__device__ __forceinline__ void pivot_zero(double bet, double x, int bad, double &v, bool &all)
+{
+    if (bad) {
+        v = zero_of(x, bet);
+        all = all && is_zero(x);
+    }
+}
+
+// (bad, bit by bit: 1/bet, and its products with t, c and d)
+static __device__ __noinline__ double3 pivot3_rare(double bet, double t, double c, double d,
+                                                   double u, double g, double w, int bad)
+{
+    bool all = !(bad & 1);
+    pivot_zero(bet, t, bad & 2, u, all);
+    pivot_zero(bet, c, bad & 4, g, all);
+    pivot_zero(bet, d, bad & 8, w, all);
+    return all ? make_double3(u, g, w) : pivot3_fp64(bet, t, c, d);
+}
+
 // u = t * (1/bet), g = c * (1/bet) and w = d * (1/bet): the rows of the
 // partitioned solves.
 __device__ __forceinline__ void pivot3(double bet, double t, double c, double d, double &u,
                                        double &g, double &w)
 {
-    bool bad;
-    const Mant y = rcp_mant(bet, bad);
+    bool bb, bt = false, bc = false, bd = false;
+    const Mant y = rcp_mant(bet, bb);
     const unsigned exps = rcp_exps(bet);
-    u = mul_mant(t, y, exps, bad);
-    g = mul_mant(c, y, exps, bad);
-    w = mul_mant(d, y, exps, bad);
-    if (bad) {
-        const double3 r = pivot3_fp64(bet, t, c, d);
+    u = mul_mant(t, y, exps, bt);
+    g = mul_mant(c, y, exps, bc);
+    w = mul_mant(d, y, exps, bd);
+    if (bb | bt | bc | bd) {
+        const double3 r = pivot3_rare(bet, t, c, d, u, g, w,
+                                      (int)bb | (int)bt << 1 | (int)bc << 2 | (int)bd << 3);
         u = r.x;
         g = r.y;
         w = r.z;
@@ -455,7 +517,7 @@ __device__ __forceinline__ double xs(double a, double b) { return __dsub_rn(a, b
 __device__ __forceinline__ double xd(double a, double b) { return div_full(a, b); }
 // xm on the integer pipes (b of ordinary size), for products that no chain
 // waits for.
-__device__ __forceinline__ double xmi(double a, double b) { return mul_full(a, b); }
+__device__ __forceinline__ double xmi(double a, double b) { return mul_full<true>(a, b); }
 
 // Selection part of Mfunc (dadi/integration_shared.c:12-14) in the
 // reference's order: gamma * 2*(h + (1.-2*h)*x) * x*(1.-x).

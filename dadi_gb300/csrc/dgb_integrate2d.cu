@@ -368,7 +368,10 @@ __device__ __forceinline__ bool k2w_leaves(int *live)
 // (longest first); to that comes what they slow each other down while all of
 // them have work.  The k with the least runs.  A kernel of its own, and asked
 // where a CTA takes its items: more code at the head of k_integrate2d_ws gave
-// its loop other registers and cost 4-6 %.
+// its loop other registers and cost 4-6 %.  For one and two warps of lines; at
+// three, where an SM holds two CTAs, 320 sets of 100 steps at 80 points would
+// gain (10.1 and 7.9 ms), but IM sets lose (400 at 70/75/80 201-208 and
+// 207-213).
 // Milliseconds with k2w_per_sm's count and so: 320 sets of 100 steps at 31
 // points 4.01 and 1.63, at 64 7.16 and 3.87; 160 such at 40/50/60 points 7.44
 // and 4.05; 320 sets of 30 to 170 steps at 31/38/45 6.13 and 5.00; IM sets,

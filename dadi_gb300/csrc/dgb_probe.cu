@@ -47,6 +47,22 @@ __global__ void k_pivot(const double *xtc, double *out, int n)
     for (int k = 0; k < 8; k++)
         out[k * (size_t)n + i] = v[k];
 }
+// t, c and d times 1/x by pivot3, c * x by mul_full<true> and, after them, on
+// doubles.
+__global__ void k_pivot3(const double *xtcd, double *out, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n)
+        return;
+    const size_t s = (size_t)n;
+    double u, g, w;
+    pivot3(xtcd[i], xtcd[s + i], xtcd[2 * s + i], xtcd[3 * s + i], u, g, w);
+    const double3 r = pivot3_fp64(xtcd[i], xtcd[s + i], xtcd[2 * s + i], xtcd[3 * s + i]);
+    const double x = xtcd[i], c = xtcd[2 * s + i];
+    const double v[8] = {u, g, w, mul_full<true>(c, x), r.x, r.y, r.z, __dmul_rn(c, x)};
+    for (int k = 0; k < 8; k++)
+        out[k * s + i] = v[k];
+}
 } // namespace dgb
 
 extern "C" int dgb_probe_fp64_fma(double *out, int blocks, int threads, int iters,
@@ -79,6 +95,19 @@ extern "C" int dgb_probe_pivot(const double *xtc, double *out, int n, void *stre
     return cudaGetLastError() == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
 }
 
+extern "C" int dgb_probe_pivot3(const double *xtcd, double *out, int n, void *stream)
+{
+    if (!xtcd || !out || n < 0)
+        return DGB_ERR_ARG;
+    if (n == 0)
+        return DGB_OK;
+    dgb::k_pivot3<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(xtcd, out, n);
+    return cudaGetLastError() == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
+}
+
 namespace dgb {
-int preload_probe() { return preload(k_fp64_fma) + preload(k_rcp) + preload(k_pivot); }
+int preload_probe()
+{
+    return preload(k_fp64_fma) + preload(k_rcp) + preload(k_pivot) + preload(k_pivot3);
+}
 } // namespace dgb

@@ -616,6 +616,9 @@ int dgb_integrate2d_noalloc(double *phi, int L, const double *xx, const double *
  * c * (1/x), t / x and c * x as the sweeps' integer arithmetic gives them,
  * then the same four as FP64 instructions give them (8 n doubles), so tests
  * can compare the bits.
+ * dgb_probe_pivot3: for xtcd = x[n], t[n], c[n], d[n] (device), out = t, c and
+ * d times 1/x as the partitioned solves form them and c * x as the delj rows
+ * do, then the same four as FP64 instructions give them (8 n doubles).
  * dgb_probe_split2d: the launch that the automatic shape of
  * dgb_batch2d_integrate and dgb_items2d_integrate (not one_per_cta) takes for
  * nwork ordered items on grids of up to Lmax points with ws_bytes of
@@ -627,6 +630,7 @@ int dgb_probe_fp64_fma(double *out, int blocks, int threads, int iters, int acti
                        void *stream);
 int dgb_probe_rcp(const double *x, double *out, int n, void *stream);
 int dgb_probe_pivot(const double *xtc, double *out, int n, void *stream);
+int dgb_probe_pivot3(const double *xtcd, double *out, int n, void *stream);
 int dgb_probe_split2d(int Lmax, long nwork, int use_delj_trick, size_t ws_bytes, int *ctas,
                       int *keep_a);
 

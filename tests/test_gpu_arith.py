@@ -62,6 +62,47 @@ def test_integer_pivot_gives_the_bits_of_the_doubles(cuda_lib, kind):
     assert same.all()
 
 
+def _same_bits(a, b):
+    return (a.view(np.int64) == b.view(np.int64)) | (np.isnan(a) & np.isnan(b))
+
+
+@pytest.mark.parametrize("kind", ["pivots", "wide", "short mantissas", "any bits"])
+def test_integer_pivot_of_the_partitioned_rows(cuda_lib, kind):
+    """The partitioned solves' three products with 1/x and the delj rows'
+    product are the FP64 instructions', bit for bit."""
+    import torch
+    from dadi_gb300 import _lib
+    n = 1 << 18
+    with np.errstate(all="ignore"):
+        x, t, c = _pivot_inputs(kind, n)
+        d = np.roll(t, 5)
+    xtcd = torch.from_numpy(np.concatenate([x, t, c, d])).cuda()
+    o = torch.empty(8 * n, dtype=torch.float64, device="cuda")
+    _lib.check(cuda_lib.dgb_probe_pivot3(_lib.dptr(xtcd), _lib.dptr(o), n,
+                                         _lib.stream_handle(torch)), "pivot3")
+    o = o.cpu().numpy()
+    assert _same_bits(o[:4 * n], o[4 * n:]).all()
+
+
+def test_integer_pivot_of_zeros(cuda_lib):
+    """Zeros of both signs in every place, against ordinary values, the ends of
+    the integers' ranges, infinities and NaN."""
+    import itertools
+    import torch
+    from dadi_gb300 import _lib
+    v = [0.0, -0.0, 1.0, -1.5, 3.7e5, -2e-7, 5e-324, 1e-310, 2.0 ** -129, 2.0 ** 128, -2.0 ** 900,
+         2.0 ** -900, np.inf, -np.inf, np.nan]
+    x, t, c, d = [np.ascontiguousarray(a) for a in np.array(list(itertools.product(v, repeat=4))).T]
+    n = len(x)
+    for call, cols in ((cuda_lib.dgb_probe_pivot, (x, t, c)),
+                       (cuda_lib.dgb_probe_pivot3, (x, t, c, d))):
+        a = torch.from_numpy(np.concatenate(cols)).cuda()
+        o = torch.empty(8 * n, dtype=torch.float64, device="cuda")
+        _lib.check(call(_lib.dptr(a), _lib.dptr(o), n, _lib.stream_handle(torch)), "pivot")
+        o = o.cpu().numpy()
+        assert _same_bits(o[:4 * n], o[4 * n:]).all()
+
+
 def test_fp64_rate_and_idle_lanes(cuda_lib):
     """The FP64 FMA rate is positive and a warp instruction with a quarter of
     its lanes active takes as long as a full one (idle lanes are not free),
