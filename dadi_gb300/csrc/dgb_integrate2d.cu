@@ -333,7 +333,9 @@ __host__ __device__ inline size_t k2w_smem_doubles(int L)
 }
 
 // Groups of W warps of a CTA: solves, factors, and (few lines, where the
-// vectors would hold up the solves) the vectors.
+// vectors would hold up the solves) the vectors.  Milliseconds of 200 steps of
+// one grid with two groups / with three: L = 31 3.61 / 3.09, 45 4.68 / 4.08, 64
+// 5.01 / 4.95, 80 6.92 / 7.22, 96 8.23 / 8.57.
 __host__ __device__ constexpr int k2w_groups(int W) { return W <= 2 ? 3 : 2; }
 
 // How much one of k CTAs of W warps of lines on an SM is slower than one alone
@@ -419,6 +421,9 @@ __global__ void __launch_bounds__(K2W_LIVE_THREADS)
     *live = best;
 }
 
+// (CTAs per SM of the launch bounds: with 4, 2 and 1 grids of 45 points, 3000
+// sets of 40 steps, take 12.0 ms and with 6, 4 and 2 10.3, against 10.2; one
+// grid alone 4.08 and 4.38 ms for 200 steps, against 4.07.)
 template <int W, bool KEEP_A, bool CHOSEN = false>
 __global__ void __launch_bounds__(32 * W * k2w_groups(W), W == 1 ? 5 : W == 2 ? 3 : 2)
     k_integrate2d_ws(K2Args A)
@@ -591,11 +596,14 @@ __global__ void __launch_bounds__(32 * W * k2w_groups(W), W == 1 ? 5 : W == 2 ? 
 // warps of lines on they fill the FP64 pipe, whatever the groups.  Every
 // operation is solve_line_delj's, so the results are bitwise the same.
 // Measured, microseconds per step of one grid with one warp for both / with
-// this kernel: L = 31 135 / 46, 60 256 / 103, 90 384 / 206, 128 544 / 359.
-constexpr __host__ __device__ int k2d_groups(int W)
-{
-    return W == 1 ? 8 : W == 2 ? 6 : W == 3 ? 5 : W == 4 ? 4 : 3;
-}
+// this kernel: L = 31 135 / 41, 60 256 / 95, 90 384 / 194, 128 544 / 361.
+//
+// Milliseconds of 100 steps of one grid with 2, 3, 4, 5, 6 groups: L = 31 5.78
+// 4.11 4.35 4.33 4.33 (8: 4.49), 60 11.8 9.80 9.52 9.68 10.4, 90 22.0 19.7 19.5
+// 21.1 22.6, 128 36.8 36.2 36.5 38.0 41.2, 150 53.5 52.7 59.3 66.2; of 40 steps
+// of 400 sets at 60 points 14.0 11.9 11.9 12.1 12.8, of 200 at 90 16.9 15.4 15.4
+// 17.0 18.3.
+constexpr __host__ __device__ int k2d_groups(int W) { return W == 2 || W == 3 ? 4 : 3; }
 
 __host__ __device__ inline size_t k2d_smem_doubles(int L)
 {
@@ -1214,7 +1222,10 @@ static int k2w_most_per_sm(int Lmax, long nwork, int sms, int fit)
 // workspace where this launch's slices are within 0.8 of the L2 cache, and
 // form it again (one more FP64 instruction a point, a third less traffic)
 // where not, whether or not the smaller slices are then within it: 152 grids
-// of 128 points 90 us a step with a, 62 without; of 100 points 46 and 51.
+// of 128 points 90 us a step with a, 62 without; of 100 points 46 and 51.  The
+// rule looks at one launch; 1000 IM sets at pts 80/90/100 in one launch per
+// grid, side by side, take 628 ms by it, 660 if all keep their a and 634 if
+// none does.
 // choose: k2w_live may choose the CTAs per SM.
 static bool k2w_plan(int Lmax, bool delj_rows, long nwork, size_t bytes, int sms, bool choose,
                      K2WPlan &p)
