@@ -330,7 +330,8 @@ __device__ void ad_step_setup(ADShared &S, ADVecs &V, const GridVecs &g, int L, 
 }
 
 // Solve all lines of axis a of the L x L row-major array u (in place), with
-// the forward or transposed vectors.
+// the forward or transposed vectors (FP64: see solve_line).
+template <bool FP64 = false>
 __device__ void ad_sweep(double *u, double *gam, int L, int a, const AxisVecs &v,
                          const AxisScalars &s, const GridVecs &g, int j0, int j1, int pu = 0)
 {
@@ -342,7 +343,7 @@ __device__ void ad_sweep(double *u, double *gam, int L, int a, const AxisVecs &v
         double W = s.mig[1 - a] * g.x[line];
         double bs = (line == j0) ? s.bcs : 0.0;
         double be = (line == j1) ? s.bce : 0.0;
-        solve_line(u + (size_t)line * sl, sp, gam + line, L, L, W, bs, be, v, s);
+        solve_line<FP64>(u + (size_t)line * sl, sp, gam + line, L, L, W, bs, be, v, s);
     }
 }
 
@@ -1151,7 +1152,11 @@ __global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs 
 // steps into the item's trajectory; phi at a segment boundary is written by
 // the next segment's CTA (its checkpoint), so no slot has two writers.  The
 // steps use ad_step_setup and ad_sweep as k_adjoint2d's own recomputation
-// does, so the trajectory is bitwise what it would recompute.
+// does, so the trajectory is bitwise what it would recompute; the solves run
+// over global memory, and on the FP64 pipe where two CTAs share an SM (three
+// schedules of 19,546 steps at pts 100/110/120: 86-92 ms on the integer pipes,
+// 58 so; one of 2,648 steps at 120 points, a third of a CTA per SM, 13.4 on the
+// FP64 pipe and 11.4 on the integer ones).
 __global__ void __launch_bounds__(AD_THREADS) k_adjoint2d_traj(ADArgs A, const long *seg_off)
 {
     extern __shared__ __align__(16) double smem[];
@@ -1164,6 +1169,7 @@ __global__ void __launch_bounds__(AD_THREADS) k_adjoint2d_traj(ADArgs A, const l
     double *gam = A.scratch + (size_t)blockIdx.x * L2max;
     const long total = seg_off[A.nwork];
     const int C = A.ckpt_every;
+    const bool full = total > gridDim.x / 2; // more than one CTA per SM has work
     for (long gs = blockIdx.x; gs < total; gs += gridDim.x) {
         int lo = 0, hi = A.nwork; // seg_off[lo] <= gs < seg_off[hi]
         while (hi - lo > 1) {
@@ -1213,6 +1219,12 @@ __global__ void __launch_bounds__(AD_THREADS) k_adjoint2d_traj(ADArgs A, const l
         const int j0 = (g.x[0] == 0.0) ? 0 : -1;
         const int j1 = (g.x[L - 1] == 1.0) ? L - 1 : -1;
         const int k0 = sgi * C, k1 = min(k0 + C, n);
+        auto sweep = [&](double *u, int a) {
+            if (full)
+                ad_sweep<true>(u, gam, L, a, V.f[a], S.ax[a], g, j0, j1);
+            else
+                ad_sweep<false>(u, gam, L, a, V.f[a], S.ax[a], g, j0, j1);
+        };
         for (size_t idx = tid; idx < LL; idx += blockDim.x)
             tphi[(size_t)k0 * LL + idx] = ck[(size_t)sgi * LL + idx];
         __syncthreads();
@@ -1231,7 +1243,7 @@ __global__ void __launch_bounds__(AD_THREADS) k_adjoint2d_traj(ADArgs A, const l
             }
             __syncthreads();
             if (!(frozen & 1)) {
-                ad_sweep(chik, gam, L, 0, V.f[0], S.ax[0], g, j0, j1);
+                sweep(chik, 0);
                 __syncthreads();
             }
             // phi_{k+1}, except at a segment boundary (the next CTA's checkpoint)
@@ -1241,7 +1253,7 @@ __global__ void __launch_bounds__(AD_THREADS) k_adjoint2d_traj(ADArgs A, const l
                     dst[idx] = chik[idx];
                 __syncthreads();
                 if (!(frozen & 2)) {
-                    ad_sweep(dst, gam, L, 1, V.f[1], S.ax[1], g, j0, j1);
+                    sweep(dst, 1);
                     __syncthreads();
                 }
             }

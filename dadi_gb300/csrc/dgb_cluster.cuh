@@ -56,18 +56,6 @@ __device__ __forceinline__ void c2_pivot3(double bet, double t, double c, double
     }
 }
 
-template <bool FP64>
-__device__ __forceinline__ void c2_pivot(double bet, double t, double c, double &u, double &g)
-{
-    if (FP64) {
-        const double inv = rcp_newton_here(bet);
-        u = t * inv;
-        g = c * inv;
-    } else {
-        pivot(bet, t, c, u, g);
-    }
-}
-
 template <bool FP64> __device__ __forceinline__ void c2_bar()
 {
     if (FP64)
@@ -165,7 +153,7 @@ __device__ __forceinline__ void c2_sweep_x(cooperative_groups::cluster_group &cl
             const double rc = -gaq * Cn;
             const double rd = fma(-gaq, Dn, fma(-alq, Dp, deq));
             const double bet = (q == 0) ? rb : fma(-ra, gq, rb);
-            c2_pivot<FP64>(bet, (q == 0) ? rd : fma(-ra, u, rd), rc, u, gq);
+            pivot_as<FP64>(bet, (q == 0) ? rd : fma(-ra, u, rd), rc, u, gq);
             gm[q] = gq;
             z[q] = u;
         }
@@ -280,7 +268,7 @@ __device__ __forceinline__ void c2_sweep_y(double *blk, int pitch, int L, int R0
             const double ra = rr[3 * C2_ROWS], rb = rr[4 * C2_ROWS];
             const double rc = rr[5 * C2_ROWS], rd = rr[6 * C2_ROWS];
             const double bet = (k == 0) ? rb : fma(-ra, gq, rb);
-            c2_pivot<FP64>(bet, (k == 0) ? rd : fma(-ra, u, rd), rc, u, gq);
+            pivot_as<FP64>(bet, (k == 0) ? rd : fma(-ra, u, rd), rc, u, gq);
             gm[k] = gq;
             z[k] = u;
         }

@@ -309,6 +309,19 @@ __device__ __forceinline__ void pivot(double bet, double t, double c, double &u,
     }
 }
 
+// The same, on the FP64 pipe if FP64.
+template <bool FP64>
+__device__ __forceinline__ void pivot_as(double bet, double t, double c, double &u, double &g)
+{
+    if (FP64) {
+        const double inv = rcp_newton_here(bet);
+        u = t * inv;
+        g = c * inv;
+    } else {
+        pivot(bet, t, c, u, g);
+    }
+}
+
 static __device__ __noinline__ double3 pivot3_fp64(double bet, double t, double c, double d)
 {
     const double inv = rcp_newton(bet);
@@ -636,13 +649,15 @@ __device__ __forceinline__ void back_substitute(TP *__restrict__ ph, int sp,
 // Thomas solve of one line, delta_j = 0.5.  Element p of the line is
 // ph[p*sp]; gam scratch element p is gm[p*gs].  W is the line's migration
 // weight, bs/be the corner boundary terms for this line (0 if none).
-template <typename TP, typename TG>
+// FP64: the pivots on the FP64 pipe (the same bits), for lines in global memory
+// on full SMs, where the rare call of the integer ones would hold up the loads.
+template <bool FP64 = false, typename TP, typename TG>
 __device__ __forceinline__ void solve_line(TP *__restrict__ ph, int sp, TG *__restrict__ gm,
                                            int gs, int L, double W, double bs, double be,
                                            const AxisVecs &v, const AxisScalars &s)
 {
     double u, g, none;
-    pivot(fma(W, s.B1s, v.B0[0]) + bs, ph[0], fma(W, v.C1[0], v.C0[0]), u, g);
+    pivot_as<FP64>(fma(W, s.B1s, v.B0[0]) + bs, ph[0], fma(W, v.C1[0], v.C0[0]), u, g);
     ph[0] = u;
     gm[gs] = g;
     // row i's coefficients and right-hand side are formed while row i - 1's
@@ -655,11 +670,11 @@ __device__ __forceinline__ void solve_line(TP *__restrict__ ph, int sp, TG *__re
         c = fma(W, v.C1[i + 1], v.C0[i + 1]);
         b0 = v.B0[i + 1];
         p = ph[(i + 1) * sp];
-        pivot(bet, t, ci, u, g);
+        pivot_as<FP64>(bet, t, ci, u, g);
         ph[i * sp] = u;
         gm[(i + 1) * gs] = g;
     }
-    pivot(fma(-a, g, fma(W, s.B1e, b0) + be), fma(-a, u, p), 1.0, u, none);
+    pivot_as<FP64>(fma(-a, g, fma(W, s.B1e, b0) + be), fma(-a, u, p), 1.0, u, none);
     ph[(L - 1) * sp] = u;
     back_substitute(ph, sp, gm, gs, L, u);
 }
