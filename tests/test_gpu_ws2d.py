@@ -153,6 +153,24 @@ def test_same_bits_where_ctas_choose_to_run(cuda_lib, L, n, spread):
     assert np.array_equal(got, want)
 
 
+def test_checkpoints_where_ctas_choose_to_run(cuda_lib):
+    """The same launch with checkpoints, from which gradients are walked back:
+    the bits of the gradients from k_integrate2d's."""
+    import torch
+    from dadi_gb300 import batch
+    p = _sets(200, 9, 5)
+    p[:, 3] *= np.linspace(0.2, 2, 200)
+    data = torch.ones(5, 5, dtype=torch.float64, device="cuda")
+    out = []
+    for threads in (0, 128):
+        eng = batch.Batch2D((31,), (4, 4))
+        eng.threads = threads
+        ll, grad, _ = eng.loglik_and_grad(p, data, scale=10.0)
+        out.append((ll.cpu().numpy(), grad.cpu().numpy()))
+    assert np.isfinite(out[1][1]).all()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
 def test_end_of_the_split_kernels_range(cuda_lib):
     """159 points are the last that the split kernels take."""
     for delj in (False, True):
