@@ -10,12 +10,13 @@ The knobs, each a real alternative the kernels implement:
 * ... or "per_grid": one persistent launch per grid size, each shaped for
   its own L (CTAs per SM, warps per CTA), on side streams so that one
   launch's tail overlaps the next;
-* gam placement — the Thomas recurrence's scratch in shared memory (fewer
-  CTAs per SM when the density already fills it) or in a per-CTA slice of
-  the workspace (more CTAs per SM, L2 traffic on the back substitution);
-* threads per CTA — 0 lets the engine run the factors of each sweep on other
-  warps than its solves where gam placement allows (2: yes, 1: no); 128 runs
-  both on four warps.
+* gam placement — 1 keeps the Thomas recurrence's scratch in shared memory
+  and runs a sweep's factors and solves on one warp; 2 puts the scratch in a
+  per-CTA slice of the workspace, through which the factors of a sweep, on
+  warps of their own, hand over to its solves (one_per_cta: on one warp, with
+  the scratch alone in the slice);
+* threads per CTA — 0 leaves that to the engine; 128 runs factors and solves
+  on the same four warps whatever the placement.
 
 `tune_batch2d` times every candidate on a sample of the batch — instances
 spread over the batch's cost distribution, so the sample has the batch's mix

@@ -29,7 +29,7 @@ struct ADNArgs {
     NDArgs nd;          // lam as nd.phi; axis, strides, table row
     const double *out;  // this sweep's forward output s_j
     const double *rhs;  // this sweep's forward input s_{j-1} (psi without injection)
-    double *gpart;      // per CTA: row_stride(P) doubles
+    double *gpart;      // per 32 lines: row_stride(P) doubles
     const double *coef; // coefficient records of the chunk from step0 (null: build inline)
     long step0;
     long rec_off;       // offset of this integration's records after the grid constants

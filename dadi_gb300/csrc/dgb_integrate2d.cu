@@ -21,9 +21,9 @@
 // per grid size with a CTA shaped for it), or one CTA per item.  Under the
 // default delta_j the factorisations of a sweep run on other warps than its
 // solves (k_integrate2d_ws), under the delj trick its coefficients
-// (k_integrate2d_delj); k_integrate2d, one warp for both, serves an explicit
-// CTA size or scratch placement, grids beyond 160 points, and callers without
-// workspace.
+// (k_integrate2d_delj), up to 159 points; k_integrate2d, one warp for both,
+// serves an explicit CTA size, the scratch in shared memory, one CTA per item,
+// larger grids, and callers without workspace.
 //
 // Reference: the time loop of Integration.two_pops (dadi/Integration.py:
 // 340-386) with implicit_2Dx / implicit_2Dy (dadi/integration2D.c:19-160).
