@@ -886,6 +886,20 @@ def run_profile_kernel(a):
             eng = batch.Batch2D(PTS_L, NS)
             eng.loglik_and_grad(draws[sel], torch.ones(41, 41, dtype=torch.float64,
                                                        device="cuda"), 1.0)
+        elif a.profile == "delj2d":
+            # 152 IM sets of 200-300 steps at pts 60 under the delj trick: one
+            # CTA per SM
+            from dadi_gb300 import integration
+            draws = im_draws(NINST, 0)
+            steps = batch.count_steps(batch.im_instances(draws))
+            sel = np.where((steps >= 200) & (steps <= 300))[0][:152]
+            eng = batch.Batch2D((60,), (20, 20))
+            saved = integration.use_delj_trick
+            try:
+                integration.use_delj_trick = True
+                eng.integrate(batch.im_instances(draws[sel]))
+            finally:
+                integration.use_delj_trick = saved
         elif a.profile == "batchnd":
             # 48 sets of the three-population growth model at pts 70 as one
             # batch (132 MB of densities, more than L2)
@@ -991,7 +1005,7 @@ def main():
     ap.add_argument("--profile", default=None,
                     choices=["epilogue", "sweep3d", "adjoint2d", "adjointnd", "batchnd",
                              "fromphind", "thomas3d", "part3d", "adjointnd_batch",
-                             "cluster2d", "adjoint2d_cluster", "grad_request"],
+                             "cluster2d", "adjoint2d_cluster", "grad_request", "delj2d"],
                     help="run a small case of another kernel for profiler captures, then exit")
     ap.add_argument("--line-solvers", action="store_true",
                     help="time the batched N-D engine's line solvers on the growth model's "
