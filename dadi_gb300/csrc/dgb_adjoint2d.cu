@@ -1152,11 +1152,16 @@ __global__ void __launch_bounds__(32 * W * ADW_GROUPS, 1) k_adjoint2d_ws(ADArgs 
 // steps into the item's trajectory; phi at a segment boundary is written by
 // the next segment's CTA (its checkpoint), so no slot has two writers.  The
 // steps use ad_step_setup and ad_sweep as k_adjoint2d's own recomputation
-// does, so the trajectory is bitwise what it would recompute; the solves run
-// over global memory, and on the FP64 pipe where two CTAs share an SM (three
-// schedules of 19,546 steps at pts 100/110/120: 86-92 ms on the integer pipes,
-// 58 so; one of 2,648 steps at 120 points, a third of a CTA per SM, 13.4 on the
-// FP64 pipe and 11.4 on the integer ones).
+// does, so the trajectory is bitwise what it would recompute.  The solves run
+// over global memory; on grids of more than AD_TRAJ_FP64_L points, where two
+// CTAs share an SM, their pivots are on the FP64 pipe (whose instructions the
+// loads of later rows pass).  Milliseconds on the integer pipes / on the FP64
+// pipe: 30 IM sets at 64 points 7.6 / 8.7, 80 10.7 / 12.4, 88 12.8 / 13.6, 96
+// 16-17 / 16.0, 104 20-26 / 18.7, 24 at 128 35-39 / 23.6, three schedules of
+// 19,546 steps at pts 100/110/120 86-92 / 58; with a third of a CTA per SM, one
+// of 2,648 steps at 120 points, 11.4 / 13.4.
+constexpr int AD_TRAJ_FP64_L = 92;
+
 __global__ void __launch_bounds__(AD_THREADS) k_adjoint2d_traj(ADArgs A, const long *seg_off)
 {
     extern __shared__ __align__(16) double smem[];
@@ -1220,7 +1225,7 @@ __global__ void __launch_bounds__(AD_THREADS) k_adjoint2d_traj(ADArgs A, const l
         const int j1 = (g.x[L - 1] == 1.0) ? L - 1 : -1;
         const int k0 = sgi * C, k1 = min(k0 + C, n);
         auto sweep = [&](double *u, int a) {
-            if (full)
+            if (full && L > AD_TRAJ_FP64_L)
                 ad_sweep<true>(u, gam, L, a, V.f[a], S.ax[a], g, j0, j1);
             else
                 ad_sweep<false>(u, gam, L, a, V.f[a], S.ax[a], g, j0, j1);
